@@ -21,11 +21,10 @@
 // and the reference QP's residual and gap measures (:2975-2994): p_res = |rp|_inf / max(1, |b|_inf),
 // d_res = |rd|_inf / max(1, |c|_inf + |Qx|_inf), gap = w'z / (1 + |objective|).
 //
-// The whole solve is one launch of one CTA: the vector passes are spread over its threads, and so
-// is the banded factorization: the columns are cut into up to 512 segments, one per thread, each an
-// interior factored as a band chain (window in registers, next column loaded ahead) plus a
-// separator of kd columns; the separators' Schur complement, block tridiagonal, is factored by one
-// thread (part_factor / part_solve below). SOVEREIGN_XBAND_SEGMENTS=1 gives the single chain.
+// The whole solve is one launch of one thread-block cluster (16 CTAs where the device can place
+// one): the vector passes are spread over all its threads, scalars are folded through distributed
+// shared memory, and K is factored and solved by odd-even block reduction (reduce_level below).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -39,10 +38,15 @@
 #include "dd.cuh"
 #include "xband.hpp"
 
+namespace cg = cooperative_groups;
+
 namespace sov {
 namespace {
 
-constexpr int kXbThreads = 512;
+constexpr int kXbThreads = 256;   // per CTA: a level's step keeps up to seven KD x KD blocks in registers
+constexpr int kXbCluster = 16;    // CTAs of the cluster (8, the portable size, where 16 cannot be placed)
+constexpr int kXbMaxLevels = 32;
+constexpr int kXbTop = 512;       // levels of at most this many blocks run in CTA 0 alone
 
 struct XbOut {
   int status, iterations, history_len, failed;
@@ -60,14 +64,21 @@ struct XbDev {
   // iterates: x and z in double-double, w in FP64
   double *xh, *xl, *zh, *zl, *w;
   // work
-  double *th, *rph, *rpl, *rd, *uh, *ul, *dxh, *dxl, *dw, *dzh, *dzl, *dwa, *dza;
-  double *Kh, *Kl;  // (kd + 1) x n: K[j][j - p] at p * n + j, overwritten by L (p >= 1) and 1 / D (p = 0)
-  // partitioned factorization: P segments, each an interior and (but the last) a separator of kd
-  int P;
-  double *Wh, *Wl;  // 2 kd x n: the interiors' spikes K_II^-1 K_IS (left kd columns, then right kd)
-  double *Ch, *Cl;  // P x 3 x kd^2: Schur contributions of each interior (to S_{s-1}, to S_s, block (s, s-1))
-  double *Th, *Tl;  // P x 2 x kd^2: separator chain factors (L_t, then D_t^-1)
-  double *Rh, *Rl;  // P x 2 x kd: the interiors' contributions to the separators' right-hand sides
+  double *th, *rph, *rpl, *rd, *rcw, *uh, *ul, *dxh, *dxl, *dw, *dzh, *dzl, *dwa, *dza;
+  // odd-even reduction: per level its block count and first slot; every array below is component
+  // major (component c of block i of level l at c * slots + off[l] + i), hi then lo parts
+  int levels, natural;
+  int size[kXbMaxLevels], off[kXbMaxLevels];
+  long long slots;
+  double *Dh, *Dl;  // diagonal blocks, lower triangle packed (r (r + 1) / 2 + c)
+  double *Bh, *Bl;  // block (i, i - 1), r * kd + c
+  double *Fh, *Fl;  // right-hand sides, kd
+  double *Lh, *Ll;  // eliminated blocks: unit lower factor (strict, r (r - 1) / 2 + c),
+  double *Ih, *Il;  //   1 / D,
+  double *Xh, *Xl;  //   L^-1 B_o (coupling to the left neighbour), r * kd + c,
+  double *Uh, *Ul;  //   L^-1 B_{o+1}' (coupling to the right neighbour),
+  double *Qh, *Ql;  //   L^-1 r_o, kd
+  int* bad;         // set on a pivot that is not positive and finite
   XbOut* out;
 };
 
@@ -77,399 +88,400 @@ __device__ __forceinline__ void st_dd(double* h, double* l, long long i, dd v) {
   l[i] = v.lo;
 }
 
-// Banded L D L' of rows [a, e) of K in place, by one thread: entries that reach left of a (the
-// coupling to the separator before the range) are neither used nor overwritten. Returns false on a
-// pivot that is not positive and finite (K = Q + A' theta A is positive definite, so only a
-// breakdown of the iterate gives one).
+// ---- odd-even block reduction ----
+// Cut into blocks of KD columns, K is block tridiagonal. A level eliminates its odd blocks: with
+// D_o = L diag(d) L' (KD x KD), X = L^-1 B_o and U = L^-1 B_{o+1}' the even neighbours get
+//   D_e -= U'd^-1 U (from the left odd block) + X'd^-1 X (from the right one),
+//   B_new = -U'd^-1 X,   r_e -= U'd^-1 q + X'd^-1 q,   q = L^-1 r_o,
+// and form the next level, half as long; the last level is one block. Back down,
+//   x_o = L'^-1 d^-1 (q - X x_{o-1} - U x_{o+1}).
+// This is the block L D L' of K in an odd-even (nested dissection) order, with the blocks factored
+// rather than inverted: as stable as the natural order (d.natural = 1, SOVEREIGN_XBAND_SEGMENTS=1,
+// runs that one on one thread). About 14 levels at n = 20002 replace chains of hundreds of
+// dependent double-double steps: what bounds a solve is the latency of one step per level.
+// One thread per even block reads both odd neighbours (the left one's factor is computed twice,
+// which costs less than a barrier between factoring and updating) and stores the right one's.
+// A level takes one cluster barrier until kXbTop blocks are left; the rest runs in CTA 0.
+// Measured (n = 20002, 81 iterations): one CTA with 512 segments and a serial separator chain
+// 300 ms, this form XXX ms.
 template <int KD>
-__device__ bool band_factor_dd(double* Kh, double* Kl, int n, int a, int e) {
-  dd L[KD + 1][KD + 1];  // L[p][q] = L(j - p, j - p - q) of the rows above
-  dd Dv[KD + 1];         // D(j - p)
-  dd Di[KD + 1];         // 1 / D(j - p)
-#pragma unroll
-  for (int p = 0; p <= KD; ++p) {
-    Dv[p] = dd_from(1.0);
-    Di[p] = dd_from(1.0);
-#pragma unroll
-    for (int q = 0; q <= KD; ++q) L[p][q] = dd_from(0.0);
-  }
-  dd row[KD + 1];  // K(j, j - p)
-#pragma unroll
-  for (int p = 0; p <= KD; ++p) row[p] = (p == 0 && a < e) ? ld_dd(Kh, Kl, a) : dd_from(0.0);
-  for (int j = a; j < e; ++j) {
-    dd next[KD + 1];
-#pragma unroll
-    for (int p = 0; p <= KD; ++p)
-      next[p] = (j + 1 < e && j + 1 - p >= a) ? ld_dd(Kh, Kl, static_cast<long long>(p) * n + j + 1) : dd_from(0.0);
-    dd l[KD + 1];
-    l[0] = dd_from(1.0);
-#pragma unroll
-    for (int p = KD; p >= 1; --p) {
-      if (j - p < a) {
-        l[p] = dd_from(0.0);
-        continue;
-      }
-      dd v = row[p];
-#pragma unroll
-      for (int q = p + 1; q <= KD; ++q)  // L(j, j-q) D(j-q) L(j-p, j-q)
-        if (j - q >= a) v = dd_sub(v, dd_mul(dd_mul(l[q], Dv[q]), L[p][q - p]));
-      l[p] = dd_mul(v, Di[p]);
-    }
-    dd d = row[0];
-#pragma unroll
-    for (int p = 1; p <= KD; ++p)
-      if (j - p >= a) d = dd_sub(d, dd_mul(dd_mul(l[p], l[p]), Dv[p]));
-    if (!(d.hi > 0.0) || !isfinite(d.hi)) return false;
-    const dd di = dd_recip(d);
-#pragma unroll
-    for (int p = 1; p <= KD; ++p)
-      if (j - p >= a) st_dd(Kh, Kl, static_cast<long long>(p) * n + j, l[p]);
-    st_dd(Kh, Kl, j, di);
-#pragma unroll
-    for (int p = KD; p >= 2; --p) {
-      Dv[p] = Dv[p - 1];
-      Di[p] = Di[p - 1];
-#pragma unroll
-      for (int q = 1; q <= KD; ++q) L[p][q] = L[p - 1][q];
-    }
-    Dv[1] = d;
-    Di[1] = di;
-#pragma unroll
-    for (int q = 1; q <= KD; ++q) L[1][q] = l[q];
-#pragma unroll
-    for (int p = 0; p <= KD; ++p) row[p] = next[p];
-  }
-  return true;
-}
-
-// K_[a,e) x = rhs with the factor above, in place in rh/rl (global indexing), one thread.
-template <int KD>
-__device__ void band_solve_dd(const double* Kh, const double* Kl, int n, int a, int e, double* rh, double* rl) {
-  dd win[KD + 1];
-#pragma unroll
-  for (int p = 0; p <= KD; ++p) win[p] = dd_from(0.0);
-  for (int j = a; j < e; ++j) {  // L y = rhs, then y / D
-    dd v = ld_dd(rh, rl, j);
-#pragma unroll
-    for (int p = 1; p <= KD; ++p)
-      if (j - p >= a) v = dd_sub(v, dd_mul(ld_dd(Kh, Kl, static_cast<long long>(p) * n + j), win[p]));
-#pragma unroll
-    for (int p = KD; p >= 2; --p) win[p] = win[p - 1];
-    win[1] = v;
-    st_dd(rh, rl, j, dd_mul(v, ld_dd(Kh, Kl, j)));
-  }
-#pragma unroll
-  for (int p = 0; p <= KD; ++p) win[p] = dd_from(0.0);
-  for (int j = e - 1; j >= a; --j) {  // L' x = v
-    dd v = ld_dd(rh, rl, j);
-#pragma unroll
-    for (int p = 1; p <= KD; ++p)
-      if (j + p < e) v = dd_sub(v, dd_mul(ld_dd(Kh, Kl, static_cast<long long>(p) * n + j + p), win[p]));
-#pragma unroll
-    for (int p = KD; p >= 2; --p) win[p] = win[p - 1];
-    win[1] = v;
-    st_dd(rh, rl, j, v);
-  }
-}
-
-// ---- partitioned factorization and solve (all threads of the CTA) ----
-// Segment s of P covers [lo_s, hi_s): its interior [lo_s, e_s) with e_s = hi_s - KD, and (but the
-// last) the separator S_s = [e_s, hi_s). Interiors couple only to the separators on either side,
-// so with the separators ordered last K = [K_II K_IS; K_SI K_SS] has a block-diagonal K_II: every
-// thread factors its own interior (band L D L'), solves for its spikes W = K_II^-1 K_IS (nonzero
-// right-hand sides only next to the separators) and forms its part of the Schur complement
-// S = K_SS - K_SI W, which is block tridiagonal with KD x KD blocks. Thread 0 factors S as a
-// chain of P - 1 blocks. A solve runs the interiors, the separator chain and the back-substitution
-// y_I - W x_S. It is the band L D L' of a symmetric permutation of K, as stable as the natural one.
-template <int KD>
-__device__ __forceinline__ void seg_range(int s, int P, int n, int& lo, int& e, int& hi) {
-  lo = static_cast<int>(static_cast<long long>(s) * n / P);
-  hi = static_cast<int>(static_cast<long long>(s + 1) * n / P);
-  e = s < P - 1 ? hi - KD : hi;
-}
-
-// K(i, j), |i - j| <= KD, from the band rows; only entries the interior factors leave intact
-// (separator rows, and interior entries that reach the previous separator) are read this way
-template <int KD>
-__device__ __forceinline__ dd k_at(const XbDev& d, int i, int j) {
-  const int hi = max(i, j), p = abs(i - j);
-  return ld_dd(d.Kh, d.Kl, static_cast<long long>(p) * d.n + hi);
-}
-
-template <int KD>
-__device__ __forceinline__ void small_inverse(dd (&A)[KD][KD], dd (&inv)[KD][KD], bool& ok) {
+__device__ __forceinline__ void load_sym(const XbDev& d, long long at, dd (&A)[KD][KD]) {
 #pragma unroll
   for (int r = 0; r < KD; ++r)
 #pragma unroll
-    for (int c = 0; c < KD; ++c) inv[r][c] = dd_from(r == c ? 1.0 : 0.0);
+    for (int c = 0; c <= r; ++c) A[r][c] = ld_dd(d.Dh, d.Dl, (r * (r + 1) / 2 + c) * d.slots + at);
+}
+
+template <int KD>
+__device__ __forceinline__ void load_full(const double* h, const double* l, long long slots, long long at,
+                                          dd (&A)[KD][KD]) {
 #pragma unroll
-  for (int k = 0; k < KD; ++k) {  // Gauss-Jordan without pivoting (A is positive definite)
-    if (!(A[k][k].hi > 0.0) || !isfinite(A[k][k].hi)) ok = false;
-    const dd ip = dd_recip(A[k][k]);
+  for (int r = 0; r < KD; ++r)
+#pragma unroll
+    for (int c = 0; c < KD; ++c) A[r][c] = ld_dd(h, l, (r * KD + c) * slots + at);
+}
+
+template <int KD>
+__device__ __forceinline__ void store_full(double* h, double* l, long long slots, long long at, const dd (&A)[KD][KD]) {
+#pragma unroll
+  for (int r = 0; r < KD; ++r)
+#pragma unroll
+    for (int c = 0; c < KD; ++c) st_dd(h, l, (r * KD + c) * slots + at, A[r][c]);
+}
+
+// A (lower triangle) -> unit lower L below the diagonal, 1 / d in inv; false on a pivot that is not
+// positive and finite (K = Q + A' theta A is positive definite: only a breakdown gives one)
+template <int KD>
+__device__ __forceinline__ bool block_ldl(dd (&A)[KD][KD], dd (&inv)[KD]) {
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < KD; ++k) {
+    const dd p = A[k][k];
+    ok = ok && p.hi > 0.0 && isfinite(p.hi);
+    inv[k] = dd_recip(p);
+    dd lk[KD];
+#pragma unroll
+    for (int r = k + 1; r < KD; ++r) lk[r] = dd_mul(A[r][k], inv[k]);
+#pragma unroll
+    for (int r = k + 1; r < KD; ++r) {
+#pragma unroll
+      for (int c = k + 1; c <= r; ++c) A[r][c] = dd_sub(A[r][c], dd_mul(lk[r], A[c][k]));
+    }
+#pragma unroll
+    for (int r = k + 1; r < KD; ++r) A[r][k] = lk[r];
+  }
+  return ok;
+}
+
+// columns of M <- L^-1 M (L unit lower in A)
+template <int KD>
+__device__ __forceinline__ void lower_solve(const dd (&A)[KD][KD], dd (&M)[KD][KD]) {
+#pragma unroll
+  for (int r = 1; r < KD; ++r)
+#pragma unroll
+    for (int k = 0; k < r; ++k)
+#pragma unroll
+      for (int c = 0; c < KD; ++c) M[r][c] = dd_sub(M[r][c], dd_mul(A[r][k], M[k][c]));
+}
+template <int KD>
+__device__ __forceinline__ void lower_solve(const dd (&A)[KD][KD], dd (&v)[KD]) {
+#pragma unroll
+  for (int r = 1; r < KD; ++r)
+#pragma unroll
+    for (int k = 0; k < r; ++k) v[r] = dd_sub(v[r], dd_mul(A[r][k], v[k]));
+}
+
+// D -= M' diag(inv) M (lower triangle), r -= M' diag(inv) q
+template <int KD>
+__device__ __forceinline__ void even_update(const dd (&M)[KD][KD], const dd (&inv)[KD], const dd (&q)[KD],
+                                            dd (&D)[KD][KD], dd (&r)[KD]) {
+#pragma unroll
+  for (int k = 0; k < KD; ++k)
+#pragma unroll
+    for (int a = 0; a < KD; ++a) {
+      const dd s = dd_mul(M[k][a], inv[k]);
+#pragma unroll
+      for (int b = 0; b <= a; ++b) D[a][b] = dd_sub(D[a][b], dd_mul(s, M[k][b]));
+      r[a] = dd_sub(r[a], dd_mul(s, q[k]));
+    }
+}
+
+template <int KD>
+__device__ __forceinline__ void load_rhs(const double* h, const double* l, long long slots, long long at, dd (&v)[KD]) {
+#pragma unroll
+  for (int k = 0; k < KD; ++k) v[k] = ld_dd(h, l, k * slots + at);
+}
+template <int KD>
+__device__ __forceinline__ void store_rhs(double* h, double* l, long long slots, long long at, const dd (&v)[KD]) {
+#pragma unroll
+  for (int k = 0; k < KD; ++k) st_dd(h, l, k * slots + at, v[k]);
+}
+
+// Level l -> l + 1 by `threads` threads from `t`: factor, next level's blocks and right-hand sides.
+template <int KD>
+__device__ void reduce_level(const XbDev& d, int l, int t, int threads) {
+  const int N = d.size[l], Nn = d.size[l + 1];
+  const long long S = d.slots, o0 = d.off[l], o1 = d.off[l + 1];
+  for (int h = t; h < Nn; h += threads) {
+    const long long e = o0 + 2 * h;
+    dd D[KD][KD], r[KD], A[KD][KD], M[KD][KD], inv[KD], q[KD];
+    load_sym<KD>(d, e, D);
+    load_rhs<KD>(d.Fh, d.Fl, S, e, r);
+    if (h > 0) {  // left odd block e - 1
+      load_sym<KD>(d, e - 1, A);
+      load_rhs<KD>(d.Fh, d.Fl, S, e - 1, q);
+      dd B[KD][KD], X[KD][KD];
+      load_full<KD>(d.Bh, d.Bl, S, e, B);
+#pragma unroll
+      for (int a = 0; a < KD; ++a)
+#pragma unroll
+        for (int b = 0; b < KD; ++b) M[a][b] = B[b][a];
+      load_full<KD>(d.Bh, d.Bl, S, e - 1, X);
+      block_ldl<KD>(A, inv);
+      lower_solve<KD>(A, M);
+      lower_solve<KD>(A, X);
+      lower_solve<KD>(A, q);
+      even_update<KD>(M, inv, q, D, r);
+#pragma unroll
+      for (int a = 0; a < KD; ++a)
+#pragma unroll
+        for (int b = 0; b < KD; ++b) {
+          dd v = dd_from(0.0);
+#pragma unroll
+          for (int k = 0; k < KD; ++k) v = dd_sub(v, dd_mul(dd_mul(M[k][a], inv[k]), X[k][b]));
+          B[a][b] = v;
+        }
+      store_full<KD>(d.Bh, d.Bl, S, o1 + h, B);
+    }
+    if (2 * h + 1 < N) {  // right odd block e + 1: its factor is stored here
+      load_sym<KD>(d, e + 1, A);
+      load_rhs<KD>(d.Fh, d.Fl, S, e + 1, q);
+      load_full<KD>(d.Bh, d.Bl, S, e + 1, M);
+      if (!block_ldl<KD>(A, inv)) atomicExch(d.bad, 1);
+      lower_solve<KD>(A, M);
+      lower_solve<KD>(A, q);
+      even_update<KD>(M, inv, q, D, r);
+      store_full<KD>(d.Xh, d.Xl, S, e + 1, M);
+      store_rhs<KD>(d.Ih, d.Il, S, e + 1, inv);
+      store_rhs<KD>(d.Qh, d.Ql, S, e + 1, q);
+#pragma unroll
+      for (int a = 1; a < KD; ++a)
+#pragma unroll
+        for (int b = 0; b < a; ++b) st_dd(d.Lh, d.Ll, (a * (a - 1) / 2 + b) * S + e + 1, A[a][b]);
+      if (2 * h + 2 < N) {
+#pragma unroll
+        for (int a = 0; a < KD; ++a)
+#pragma unroll
+          for (int b = 0; b < KD; ++b) M[a][b] = ld_dd(d.Bh, d.Bl, (b * KD + a) * S + e + 2);
+        lower_solve<KD>(A, M);
+        store_full<KD>(d.Uh, d.Ul, S, e + 1, M);
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < KD; ++a)
+#pragma unroll
+      for (int b = 0; b <= a; ++b) st_dd(d.Dh, d.Dl, (a * (a + 1) / 2 + b) * S + o1 + h, D[a][b]);
+    store_rhs<KD>(d.Fh, d.Fl, S, o1 + h, r);
+  }
+}
+
+template <int KD>
+__device__ __forceinline__ void load_lower(const XbDev& d, long long at, dd (&A)[KD][KD]) {
+#pragma unroll
+  for (int a = 1; a < KD; ++a)
+#pragma unroll
+    for (int b = 0; b < a; ++b) A[a][b] = ld_dd(d.Lh, d.Ll, (a * (a - 1) / 2 + b) * d.slots + at);
+}
+
+// r -= M' diag(inv) q with M, inv of the factored block `at`, from h / l
+template <int KD>
+__device__ __forceinline__ void rhs_update(const XbDev& d, const double* Mh, const double* Ml, long long at,
+                                           const dd (&q)[KD], dd (&r)[KD]) {
+#pragma unroll
+  for (int k = 0; k < KD; ++k) {
+    const dd w = dd_mul(q[k], ld_dd(d.Ih, d.Il, k * d.slots + at));
+#pragma unroll
+    for (int a = 0; a < KD; ++a) r[a] = dd_sub(r[a], dd_mul(ld_dd(Mh, Ml, (k * KD + a) * d.slots + at), w));
+  }
+}
+
+// The right-hand side alone down one level, with the factor reduce_level left.
+template <int KD>
+__device__ void forward_level(const XbDev& d, int l, int t, int threads) {
+  const int N = d.size[l], Nn = d.size[l + 1];
+  const long long S = d.slots, o0 = d.off[l], o1 = d.off[l + 1];
+  for (int h = t; h < Nn; h += threads) {
+    const long long e = o0 + 2 * h;
+    dd r[KD], q[KD], A[KD][KD];
+    load_rhs<KD>(d.Fh, d.Fl, S, e, r);
+    if (h > 0) {
+      load_rhs<KD>(d.Fh, d.Fl, S, e - 1, q);
+      load_lower<KD>(d, e - 1, A);
+      lower_solve<KD>(A, q);
+      rhs_update<KD>(d, d.Uh, d.Ul, e - 1, q, r);
+    }
+    if (2 * h + 1 < N) {
+      load_rhs<KD>(d.Fh, d.Fl, S, e + 1, q);
+      load_lower<KD>(d, e + 1, A);
+      lower_solve<KD>(A, q);
+      rhs_update<KD>(d, d.Xh, d.Xl, e + 1, q, r);
+      store_rhs<KD>(d.Qh, d.Ql, S, e + 1, q);
+    }
+    store_rhs<KD>(d.Fh, d.Fl, S, o1 + h, r);
+  }
+}
+
+// v <- L'^-1 diag(inv) v
+template <int KD>
+__device__ __forceinline__ void upper_solve(const dd (&A)[KD][KD], const dd (&inv)[KD], dd (&v)[KD]) {
+#pragma unroll
+  for (int k = KD - 1; k >= 0; --k) {
+    v[k] = dd_mul(v[k], inv[k]);
+#pragma unroll
+    for (int a = k + 1; a < KD; ++a) v[k] = dd_sub(v[k], dd_mul(A[a][k], v[a]));
+  }
+}
+
+// The odd blocks of level l from their even neighbours; block i of level l is block i << l of the
+// matrix, and solutions go straight to their place in dx.
+template <int KD>
+__device__ void backward_level(const XbDev& d, int l, int t, int threads) {
+  const int N = d.size[l], odd = N / 2;
+  const long long S = d.slots, o0 = d.off[l];
+  for (int h = t; h < odd; h += threads) {
+    const int i = 2 * h + 1;
+    const long long at = o0 + i;
+    dd v[KD], inv[KD], A[KD][KD];
+    load_rhs<KD>(d.Qh, d.Ql, S, at, v);
+    load_rhs<KD>(d.Ih, d.Il, S, at, inv);
+    load_lower<KD>(d, at, A);
+    const long long c0 = static_cast<long long>(i - 1) * KD << l;
 #pragma unroll
     for (int c = 0; c < KD; ++c) {
-      A[k][c] = dd_mul(A[k][c], ip);
-      inv[k][c] = dd_mul(inv[k][c], ip);
-    }
+      const dd x = ld_dd(d.dxh, d.dxl, c0 + c);
 #pragma unroll
-    for (int r = 0; r < KD; ++r) {
-      if (r == k) continue;
-      const dd f = A[r][k];
+      for (int k = 0; k < KD; ++k) v[k] = dd_sub(v[k], dd_mul(ld_dd(d.Xh, d.Xl, (k * KD + c) * S + at), x));
+    }
+    if (i + 1 < N) {
+      const long long c1 = static_cast<long long>(i + 1) * KD << l;
 #pragma unroll
       for (int c = 0; c < KD; ++c) {
-        A[r][c] = dd_sub(A[r][c], dd_mul(f, A[k][c]));
-        inv[r][c] = dd_sub(inv[r][c], dd_mul(f, inv[k][c]));
+        const dd x = ld_dd(d.dxh, d.dxl, c1 + c);
+#pragma unroll
+        for (int k = 0; k < KD; ++k) v[k] = dd_sub(v[k], dd_mul(ld_dd(d.Uh, d.Ul, (k * KD + c) * S + at), x));
       }
     }
+    upper_solve<KD>(A, inv, v);
+    const long long ci = static_cast<long long>(i) * KD << l;
+#pragma unroll
+    for (int k = 0; k < KD; ++k) st_dd(d.dxh, d.dxl, ci + k, v[k]);
   }
 }
 
+// The one block of the last level.
 template <int KD>
-__device__ void part_factor(const XbDev& d, int* bad) {
-  const int P = d.P, n = d.n, s = threadIdx.x;
-  constexpr int KK = KD * KD;
-  if (s < P) {
-    int lo, e, hi;
-    seg_range<KD>(s, P, n, lo, e, hi);
-    if (!band_factor_dd<KD>(d.Kh, d.Kl, n, lo, e)) {
-      atomicExch(bad, 1);
+__device__ void solve_last(const XbDev& d, bool factor) {
+  const long long at = d.off[d.levels - 1];
+  dd A[KD][KD], inv[KD], v[KD];
+  load_rhs<KD>(d.Fh, d.Fl, d.slots, at, v);
+  if (factor) {
+    load_sym<KD>(d, at, A);
+    if (!block_ldl<KD>(A, inv)) atomicExch(d.bad, 1);
+    store_rhs<KD>(d.Ih, d.Il, d.slots, at, inv);
+#pragma unroll
+    for (int a = 1; a < KD; ++a)
+#pragma unroll
+      for (int b = 0; b < a; ++b) st_dd(d.Lh, d.Ll, (a * (a - 1) / 2 + b) * d.slots + at, A[a][b]);
+  } else {
+    load_lower<KD>(d, at, A);
+    load_rhs<KD>(d.Ih, d.Il, d.slots, at, inv);
+  }
+  lower_solve<KD>(A, v);
+  upper_solve<KD>(A, inv, v);
+#pragma unroll
+  for (int k = 0; k < KD; ++k) st_dd(d.dxh, d.dxl, k, v[k]);
+}
+
+// The natural order on one thread: block i eliminated into block i + 1.
+template <int KD>
+__device__ void solve_natural(const XbDev& d, bool factor) {
+  const int N = d.size[0];
+  const long long S = d.slots;
+  dd r[KD], D[KD][KD];
+  load_rhs<KD>(d.Fh, d.Fl, S, 0, r);
+  if (factor) load_sym<KD>(d, 0, D);
+  for (int i = 0; i < N; ++i) {
+    dd M[KD][KD], inv[KD], q[KD], A[KD][KD];
+#pragma unroll
+    for (int k = 0; k < KD; ++k) q[k] = r[k];
+    if (factor) {
+#pragma unroll
+      for (int a = 0; a < KD; ++a)
+#pragma unroll
+        for (int b = 0; b <= a; ++b) A[a][b] = D[a][b];
+      if (!block_ldl<KD>(A, inv)) atomicExch(d.bad, 1);
+      store_rhs<KD>(d.Ih, d.Il, S, i, inv);
+#pragma unroll
+      for (int a = 1; a < KD; ++a)
+#pragma unroll
+        for (int b = 0; b < a; ++b) st_dd(d.Lh, d.Ll, (a * (a - 1) / 2 + b) * S + i, A[a][b]);
     } else {
-      for (int c = 0; c < 2 * KD; ++c) {  // spikes
-        const bool left = c < KD;
-        if ((left && s == 0) || (!left && s == P - 1)) continue;
-        const int sep = left ? lo - KD + c : e + (c - KD);
-        double* wh = d.Wh + static_cast<long long>(c) * n;
-        double* wl = d.Wl + static_cast<long long>(c) * n;
-        for (int j = lo; j < e; ++j) st_dd(wh, wl, j, abs(j - sep) <= KD ? k_at<KD>(d, j, sep) : dd_from(0.0));
-        band_solve_dd<KD>(d.Kh, d.Kl, n, lo, e, wh, wl);
-      }
-      for (int which = 0; which < 3; ++which) {  // Schur contributions
-        if ((which == 0 && s == 0) || (which == 1 && s == P - 1) || (which == 2 && (s == 0 || s == P - 1))) continue;
+      load_lower<KD>(d, i, A);
+    }
+    lower_solve<KD>(A, q);
+    store_rhs<KD>(d.Qh, d.Ql, S, i, q);
+    if (i + 1 == N) break;
+    load_rhs<KD>(d.Fh, d.Fl, S, i + 1, r);
+    if (factor) {
+      load_sym<KD>(d, i + 1, D);
 #pragma unroll
-        for (int r = 0; r < KD; ++r) {
-          const int sep = which == 0 ? lo - KD + r : e + r;
-          const int j0 = which == 0 ? lo : max(lo, sep - KD), j1 = which == 0 ? min(e, sep + KD + 1) : e;
+      for (int a = 0; a < KD; ++a)
 #pragma unroll
-          for (int c = 0; c < KD; ++c) {
-            const int col = which == 1 ? KD + c : c;
-            dd acc = dd_from(0.0);
-            for (int j = j0; j < j1; ++j)
-              acc = dd_add(acc, dd_mul(k_at<KD>(d, sep, j), ld_dd(d.Wh + static_cast<long long>(col) * n,
-                                                                  d.Wl + static_cast<long long>(col) * n, j)));
-            st_dd(d.Ch, d.Cl, (static_cast<long long>(s) * 3 + which) * KK + r * KD + c, dd_neg(acc));
-          }
-        }
-      }
+        for (int b = 0; b < KD; ++b) M[a][b] = ld_dd(d.Bh, d.Bl, (b * KD + a) * S + i + 1);
+      lower_solve<KD>(A, M);
+      even_update<KD>(M, inv, q, D, r);
+      store_full<KD>(d.Uh, d.Ul, S, i, M);
+    } else {
+      rhs_update<KD>(d, d.Uh, d.Ul, i, q, r);
     }
   }
-  __syncthreads();
-  // the separators' diagonal blocks A_t = K(S_t, S_t) + the Schur parts of both neighbouring
-  // interiors, formed in parallel (into the slot of interior t's right contribution)
-  if (s < P - 1 && !*bad) {
-    int lo, e, hi;
-    seg_range<KD>(s, P, n, lo, e, hi);
+  dd x[KD];
+  for (int i = N - 1; i >= 0; --i) {
+    dd v[KD], inv[KD], A[KD][KD];
+    load_rhs<KD>(d.Qh, d.Ql, S, i, v);
+    load_rhs<KD>(d.Ih, d.Il, S, i, inv);
+    load_lower<KD>(d, i, A);
+    if (i + 1 < N)
 #pragma unroll
-    for (int r = 0; r < KD; ++r)
+      for (int c = 0; c < KD; ++c)
 #pragma unroll
-      for (int c = 0; c < KD; ++c) {
-        const long long at = (static_cast<long long>(s) * 3 + 1) * KK + r * KD + c;
-        st_dd(d.Ch, d.Cl, at,
-              dd_add(dd_add(k_at<KD>(d, e + r, e + c), ld_dd(d.Ch, d.Cl, at)),
-                     ld_dd(d.Ch, d.Cl, (static_cast<long long>(s + 1) * 3 + 0) * KK + r * KD + c)));
-      }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0 && P > 1 && !*bad) {  // block tridiagonal L D L' of S, one chain
-    bool ok = true;
-    dd Dprev[KD][KD], An[KD][KD], Bn[KD][KD];
+        for (int k = 0; k < KD; ++k) v[k] = dd_sub(v[k], dd_mul(ld_dd(d.Uh, d.Ul, (k * KD + c) * S + i), x[c]));
+    upper_solve<KD>(A, inv, v);
 #pragma unroll
-    for (int r = 0; r < KD; ++r)
-#pragma unroll
-      for (int c = 0; c < KD; ++c) {
-        An[r][c] = ld_dd(d.Ch, d.Cl, 1 * KK + r * KD + c);
-        Bn[r][c] = dd_from(0.0);
-      }
-    for (int t = 0; t < P - 1; ++t) {
-      dd A[KD][KD], B[KD][KD];
-#pragma unroll
-      for (int r = 0; r < KD; ++r)
-#pragma unroll
-        for (int c = 0; c < KD; ++c) {
-          A[r][c] = An[r][c];
-          B[r][c] = Bn[r][c];
-        }
-      if (t + 1 < P - 1)  // the next step's blocks, loaded while this one computes
-#pragma unroll
-        for (int r = 0; r < KD; ++r)
-#pragma unroll
-          for (int c = 0; c < KD; ++c) {
-            An[r][c] = ld_dd(d.Ch, d.Cl, (static_cast<long long>(t + 1) * 3 + 1) * KK + r * KD + c);
-            Bn[r][c] = ld_dd(d.Ch, d.Cl, (static_cast<long long>(t + 1) * 3 + 2) * KK + r * KD + c);
-          }
-      if (t >= 1) {
-        dd L[KD][KD];
-#pragma unroll
-        for (int r = 0; r < KD; ++r)
-#pragma unroll
-          for (int c = 0; c < KD; ++c) {
-            dd v = dd_from(0.0);
-#pragma unroll
-            for (int q = 0; q < KD; ++q) v = dd_add(v, dd_mul(B[r][q], Dprev[q][c]));
-            L[r][c] = v;
-            st_dd(d.Th, d.Tl, (static_cast<long long>(t) * 2 + 0) * KK + r * KD + c, v);
-          }
-#pragma unroll
-        for (int r = 0; r < KD; ++r)
-#pragma unroll
-          for (int c = 0; c < KD; ++c) {
-            dd v = A[r][c];
-#pragma unroll
-            for (int q = 0; q < KD; ++q) v = dd_sub(v, dd_mul(L[r][q], B[c][q]));
-            A[r][c] = v;
-          }
-      }
-      small_inverse<KD>(A, Dprev, ok);
-#pragma unroll
-      for (int r = 0; r < KD; ++r)
-#pragma unroll
-        for (int c = 0; c < KD; ++c) st_dd(d.Th, d.Tl, (static_cast<long long>(t) * 2 + 1) * KK + r * KD + c, Dprev[r][c]);
+    for (int k = 0; k < KD; ++k) {
+      x[k] = v[k];
+      st_dd(d.dxh, d.dxl, static_cast<long long>(i) * KD + k, v[k]);
     }
-    if (!ok) atomicExch(bad, 1);
   }
-  __syncthreads();
 }
 
-// K x = rhs in place in xh/xl with the partitioned factor.
+// K dx = r with r in level 0 of F: with `factor`, K (level 0 of D and B) is factored on the way
+// down, else the factor of the last such call is used. Called by the whole cluster after a barrier;
+// ends with one.
 template <int KD>
-__device__ void part_solve(const XbDev& d, double* xh, double* xl) {
-  const int P = d.P, n = d.n, s = threadIdx.x;
-  constexpr int KK = KD * KD;
-  if (s < P) {
-    int lo, e, hi;
-    seg_range<KD>(s, P, n, lo, e, hi);
-    band_solve_dd<KD>(d.Kh, d.Kl, n, lo, e, xh, xl);  // y_I
-#pragma unroll
-    for (int side = 0; side < 2; ++side) {  // K(S, I_s) y_I onto S_{s-1} (side 0) and S_s (side 1)
-      if ((side == 0 && s == 0) || (side == 1 && s == P - 1)) continue;
-#pragma unroll
-      for (int r = 0; r < KD; ++r) {
-        const int sep = side == 0 ? lo - KD + r : e + r;
-        const int j0 = side == 0 ? lo : max(lo, sep - KD), j1 = side == 0 ? min(e, sep + KD + 1) : e;
-        dd acc = dd_from(0.0);
-        for (int j = j0; j < j1; ++j) acc = dd_add(acc, dd_mul(k_at<KD>(d, sep, j), ld_dd(xh, xl, j)));
-        st_dd(d.Rh, d.Rl, (static_cast<long long>(s) * 2 + side) * KD + r, acc);
-      }
+__device__ void band_newton(const XbDev& d, bool factor, int t, int threads) {
+  cg::cluster_group cluster = cg::this_cluster();
+  if (d.natural) {
+    if (t == 0) solve_natural<KD>(d, factor);
+    cluster.sync();
+    return;
+  }
+  int l = 0;
+  for (; d.size[l] > kXbTop; ++l) {
+    if (factor) reduce_level<KD>(d, l, t, threads);
+    else forward_level<KD>(d, l, t, threads);
+    cluster.sync();
+  }
+  if (cluster.block_rank() == 0) {
+    const int tt = threadIdx.x;
+    int u = l;
+    for (; u + 1 < d.levels; ++u) {
+      if (factor) reduce_level<KD>(d, u, tt, kXbThreads);
+      else forward_level<KD>(d, u, tt, kXbThreads);
+      __syncthreads();
+    }
+    if (tt == 0) solve_last<KD>(d, factor);
+    __syncthreads();
+    for (--u; u >= l; --u) {
+      backward_level<KD>(d, u, tt, kXbThreads);
+      __syncthreads();
     }
   }
-  __syncthreads();
-  // separators' right-hand sides less the interiors' contributions, in parallel
-  if (s < P - 1) {
-    int lo, e, hi;
-    seg_range<KD>(s, P, n, lo, e, hi);
-#pragma unroll
-    for (int r = 0; r < KD; ++r)
-      st_dd(xh, xl, e + r,
-            dd_sub(dd_sub(ld_dd(xh, xl, e + r), ld_dd(d.Rh, d.Rl, (static_cast<long long>(s) * 2 + 1) * KD + r)),
-                   ld_dd(d.Rh, d.Rl, (static_cast<long long>(s + 1) * 2 + 0) * KD + r)));
+  cluster.sync();
+  for (--l; l >= 0; --l) {
+    backward_level<KD>(d, l, t, threads);
+    cluster.sync();
   }
-  __syncthreads();
-  if (threadIdx.x == 0 && P > 1) {  // forward chain z_t = r_t - L_t z_{t-1}, in the separator slots
-    dd z[KD], rn[KD], Ln[KD][KD];
-    {
-      int lo, e, hi;
-      seg_range<KD>(0, P, n, lo, e, hi);
-#pragma unroll
-      for (int r = 0; r < KD; ++r) z[r] = ld_dd(xh, xl, e + r);  // z_0 = r_0
-    }
-    for (int t = 1; t < P - 1; ++t) {
-      int lo, e, hi;
-      seg_range<KD>(t, P, n, lo, e, hi);
-#pragma unroll
-      for (int r = 0; r < KD; ++r) {
-        rn[r] = ld_dd(xh, xl, e + r);
-#pragma unroll
-        for (int c = 0; c < KD; ++c) Ln[r][c] = ld_dd(d.Th, d.Tl, (static_cast<long long>(t) * 2 + 0) * KK + r * KD + c);
-      }
-      dd zn[KD];
-#pragma unroll
-      for (int r = 0; r < KD; ++r) {
-        dd v = rn[r];
-#pragma unroll
-        for (int c = 0; c < KD; ++c) v = dd_sub(v, dd_mul(Ln[r][c], z[c]));
-        zn[r] = v;
-      }
-#pragma unroll
-      for (int r = 0; r < KD; ++r) {
-        z[r] = zn[r];
-        st_dd(xh, xl, e + r, zn[r]);
-      }
-    }
-  }
-  __syncthreads();
-  if (s < P - 1) {  // w_t = D_t^-1 z_t, in parallel
-    int lo, e, hi;
-    seg_range<KD>(s, P, n, lo, e, hi);
-    dd z[KD];
-#pragma unroll
-    for (int c = 0; c < KD; ++c) z[c] = ld_dd(xh, xl, e + c);
-#pragma unroll
-    for (int r = 0; r < KD; ++r) {
-      dd v = dd_from(0.0);
-#pragma unroll
-      for (int c = 0; c < KD; ++c) v = dd_add(v, dd_mul(ld_dd(d.Th, d.Tl, (static_cast<long long>(s) * 2 + 1) * KK + r * KD + c), z[c]));
-      st_dd(xh, xl, e + r, v);
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0 && P > 2) {  // backward chain x_t = w_t - L_{t+1}' x_{t+1}
-    dd xn[KD];
-    {
-      int lo, e, hi;
-      seg_range<KD>(P - 2, P, n, lo, e, hi);
-#pragma unroll
-      for (int r = 0; r < KD; ++r) xn[r] = ld_dd(xh, xl, e + r);
-    }
-    for (int t = P - 3; t >= 0; --t) {
-      int lo, e, hi;
-      seg_range<KD>(t, P, n, lo, e, hi);
-      dd w[KD], Lt[KD][KD];
-#pragma unroll
-      for (int r = 0; r < KD; ++r) {
-        w[r] = ld_dd(xh, xl, e + r);
-#pragma unroll
-        for (int c = 0; c < KD; ++c) Lt[r][c] = ld_dd(d.Th, d.Tl, (static_cast<long long>(t + 1) * 2 + 0) * KK + c * KD + r);
-      }
-#pragma unroll
-      for (int r = 0; r < KD; ++r)
-#pragma unroll
-        for (int c = 0; c < KD; ++c) w[r] = dd_sub(w[r], dd_mul(Lt[r][c], xn[c]));
-#pragma unroll
-      for (int r = 0; r < KD; ++r) {
-        st_dd(xh, xl, e + r, w[r]);
-        xn[r] = w[r];
-      }
-    }
-  }
-  __syncthreads();
-  if (s < P && P > 1) {  // x_I = y_I - W_left x_S(s-1) - W_right x_S(s)
-    int lo, e, hi;
-    seg_range<KD>(s, P, n, lo, e, hi);
-    dd xs[2 * KD];
-#pragma unroll
-    for (int c = 0; c < 2 * KD; ++c) {
-      const bool left = c < KD;
-      xs[c] = ((left && s == 0) || (!left && s == P - 1)) ? dd_from(0.0) : ld_dd(xh, xl, left ? lo - KD + c : e + (c - KD));
-    }
-    for (int j = lo; j < e; ++j) {
-      dd v = ld_dd(xh, xl, j);
-#pragma unroll
-      for (int c = 0; c < 2 * KD; ++c)
-        if (xs[c].hi != 0.0 || xs[c].lo != 0.0)
-          v = dd_sub(v, dd_mul(ld_dd(d.Wh + static_cast<long long>(c) * n, d.Wl + static_cast<long long>(c) * n, j), xs[c]));
-      st_dd(xh, xl, j, v);
-    }
-  }
-  __syncthreads();
 }
 
 // (A v)_r in double-double
@@ -486,29 +498,74 @@ __device__ __forceinline__ dd col_dot(const XbDev& d, int j, const double* uh, c
   return s;
 }
 
+// Cluster-wide reduction of NV values (ops: 0 sum, 1 max, 2 min): every CTA's result is written to
+// all CTAs' shared memory, and after one cluster barrier every thread folds them in rank order.
+// Two buffers taken in turn: a buffer is written again only after a later barrier.
+struct ClusterRed {
+  double v[2][4][kXbCluster];
+};
+template <int NV>
+__device__ __forceinline__ void cluster_reduce(double (&v)[NV], const int (&ops)[NV], double* red, ClusterRed& cr,
+                                               int& turn) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ctas = cluster.num_blocks();
+  block_reduce<NV>(v, ops, red);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) red[k] = v[k];
+  __syncthreads();
+  if (static_cast<int>(threadIdx.x) < ctas) {
+    ClusterRed* other = cluster.map_shared_rank(&cr, threadIdx.x);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) other->v[turn][k][cluster.block_rank()] = red[k];
+  }
+  cluster.sync();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    double acc = cr.v[turn][k][0];
+    for (int c = 1; c < ctas; ++c) {
+      const double u = cr.v[turn][k][c];
+      acc = ops[k] == 0 ? acc + u : ops[k] == 1 ? fmax(acc, u) : fmin(acc, u);
+    }
+    v[k] = acc;
+  }
+  turn ^= 1;
+}
+
 template <int KD>
-__global__ void __launch_bounds__(kXbThreads, 1) k_xband_ipm(XbDev d) {
+__global__ void __launch_bounds__(kXbThreads, 1) k_xband_ipm(const __grid_constant__ XbDev d) {
   __shared__ double red[4 * 32];
-  __shared__ double s_mu, s_sigma, s_alpha_p, s_alpha_d;
-  __shared__ int s_stop, s_bad;
-  const int tid = threadIdx.x;
+  __shared__ ClusterRed cr;
+  cg::cluster_group cluster = cg::this_cluster();
+  int turn = 0;
+  const int threads = static_cast<int>(cluster.num_blocks()) * kXbThreads;
+  const int tid = static_cast<int>(cluster.block_rank()) * kXbThreads + static_cast<int>(threadIdx.x);
   const int n = d.n, m = d.m;
   const double inf = INFINITY;
   // the reference QP stops at its tolerances; this path goes two decades further (cheap in
   // double-double) so that its objective meets the exact structured answer to 1e-8
   const double ftol = d.feas_tol * 1e-2, otol = d.opt_tol * 1e-2;
+  // every CTA runs (its shared memory can be written) before the first remote store
+  cluster.sync();
   int it = 0;
   for (;; ++it) {
-    // ---- residuals, mu, objective ----
+    // ---- residuals, mu, objective; theta and the predictor's u = rc / w + theta rp ----
     double v[4] = {0.0, 0.0, 0.0, 0.0};  // max |rp|, max |rd|, max |Qx|, w'z
-    for (int r = tid; r < m; r += kXbThreads) {
-      const dd rp = dd_add_d(dd_add_d(row_dot(d, r, d.xh, d.xl), -d.w[r]), -d.b[r]);
+    for (int r = tid; r < m; r += threads) {
+      const double w = d.w[r], z = d.zh[r], th = z / w;
+      const dd rp = dd_add_d(dd_add_d(row_dot(d, r, d.xh, d.xl), -w), -d.b[r]);
       st_dd(d.rph, d.rpl, r, rp);
+      // rc / w is FP64: the direction has to take this very value again, or its error (1e-16 of z,
+      // which reaches 1e7) stays in the dual residual
+      const double q = w * z / w;
+      d.th[r] = th;
+      d.rcw[r] = q;
+      st_dd(d.uh, d.ul, r, dd_add_d(dd_mul_d(rp, th), q));
       v[0] = fmax(v[0], fabs(rp.hi));
-      v[3] += d.w[r] * d.zh[r];
+      v[3] += w * z;
     }
     double objp = 0.0;
-    for (int j = tid; j < n; j += kXbThreads) {
+    for (int j = tid; j < n; j += threads) {
       const dd qx = dd_mul_d(ld_dd(d.xh, d.xl, j), d.q[j]);
       const dd rd = dd_sub(dd_add_d(qx, d.c[j]), col_dot(d, j, d.zh, d.zl));
       d.rd[j] = rd.hi;
@@ -517,16 +574,28 @@ __global__ void __launch_bounds__(kXbThreads, 1) k_xband_ipm(XbDev d) {
       objp += d.c[j] * d.xh[j] + 0.5 * d.q[j] * d.xh[j] * d.xh[j];
     }
     const int ops4[4] = {1, 1, 1, 0};
-    block_reduce<4>(v, ops4, red);
+    cluster_reduce<4>(v, ops4, red, cr, turn);
     double o1[1] = {objp};
     const int ops1[1] = {0};
-    block_reduce<1>(o1, ops1, red);
+    cluster_reduce<1>(o1, ops1, red, cr, turn);
+    // every thread holds the same sums, so the whole cluster takes the same decision
+    const double mu = v[3] / m;
+    const double obj = o1[0] + d.obj_constant;
+    const double p_res = v[0] / d.bnorm;
+    const double d_res = v[1] / fmax(1.0, d.cnorm + v[2]);
+    const double gap = v[3] / (1.0 + fabs(obj));
+    int status = -1, failed = 0;
+    if (!isfinite(mu) || !isfinite(p_res) || !isfinite(d_res)) {
+      status = SOV_ERROR;
+      failed = 1;
+    } else if (p_res <= ftol && d_res <= ftol && gap <= otol) {
+      status = SOV_OPTIMAL;
+    } else if (it >= d.max_iter) {
+      // at the limit the reference QP's own tolerances decide; otherwise ERROR without an
+      // objective, as its failure exits publish (qp_interior_point.cpp:3042-3048, :3112-3115)
+      status = (p_res <= d.feas_tol && d_res <= d.feas_tol && gap <= d.opt_tol) ? SOV_OPTIMAL : SOV_ERROR;
+    }
     if (tid == 0) {
-      const double mu = v[3] / m;
-      const double obj = o1[0] + d.obj_constant;
-      const double p_res = v[0] / d.bnorm;
-      const double d_res = v[1] / fmax(1.0, d.cnorm + v[2]);
-      const double gap = v[3] / (1.0 + fabs(obj));
       XbOut* o = d.out;
       o->p_res = p_res;
       o->d_res = d_res;
@@ -541,119 +610,117 @@ __global__ void __launch_bounds__(kXbThreads, 1) k_xband_ipm(XbDev d) {
         o->mu_hist[h] = mu;
         o->obj_hist[h] = obj;
       }
-      s_mu = mu;
-      s_stop = 0;
-      if (!isfinite(mu) || !isfinite(p_res) || !isfinite(d_res)) {
-        o->status = SOV_ERROR;
-        o->failed = 1;
-        s_stop = 1;
-      } else if (p_res <= ftol && d_res <= ftol && gap <= otol) {
-        o->status = SOV_OPTIMAL;
-        s_stop = 1;
-      } else if (it >= d.max_iter) {
-        // at the limit the reference QP's own tolerances decide; otherwise ERROR without an
-        // objective, as its failure exits publish (qp_interior_point.cpp:3042-3048, :3112-3115)
-        o->status = (p_res <= d.feas_tol && d_res <= d.feas_tol && gap <= d.opt_tol) ? SOV_OPTIMAL : SOV_ERROR;
-        s_stop = 1;
+      if (status >= 0) {
+        o->status = status;
+        o->failed = failed;
       }
     }
-    __syncthreads();
-    if (s_stop) break;
-    // ---- K = Q + A' theta A, double-double ----
-    for (int r = tid; r < m; r += kXbThreads) d.th[r] = d.zh[r] / d.w[r];
-    __syncthreads();
-    for (int j = tid; j < n; j += kXbThreads) {
+    if (status >= 0) break;
+    // ---- K = Q + A' theta A in double-double into level 0's blocks, predictor's rhs = -rd - A'u ----
+    for (int j = tid; j < d.size[0] * KD; j += threads) {
+      const int blk = j / KD, jr = j - blk * KD;
       dd acc[KD + 1];
 #pragma unroll
       for (int p = 0; p <= KD; ++p) acc[p] = dd_from(0.0);
-      acc[0] = dd_from(d.q[j]);
-      for (int e = d.col_ptr[j]; e < d.col_ptr[j + 1]; ++e) {
-        const int r = d.row_idx[e];
-        const double a = d.col_val[e], t = d.th[r];
-        for (int f = d.row_ptr[r]; f < d.row_ptr[r + 1]; ++f) {
-          const int k = d.col_idx[f];
-          const int p = j - k;
-          if (p < 0 || p > KD) continue;
-          const dd prod = dd_mul_d(two_prod(a, d.row_val[f]), t);
+      dd rhs = dd_from(0.0);
+      if (j < n) {
+        acc[0] = dd_from(d.q[j]);
+        dd au = dd_from(0.0);
+        for (int e = d.col_ptr[j]; e < d.col_ptr[j + 1]; ++e) {
+          const int r = d.row_idx[e];
+          const double a = d.col_val[e], t = d.th[r];
+          au = dd_add(au, dd_mul_d(ld_dd(d.uh, d.ul, r), a));
+          for (int f = d.row_ptr[r]; f < d.row_ptr[r + 1]; ++f) {
+            const int k = d.col_idx[f];
+            const int p = j - k;
+            if (p < 0 || p > KD) continue;
+            const dd prod = dd_mul_d(two_prod(a, d.row_val[f]), t);
 #pragma unroll
-          for (int q = 0; q <= KD; ++q)
-            if (q == p) acc[q] = dd_add(acc[q], prod);
+            for (int q = 0; q <= KD; ++q)
+              if (q == p) acc[q] = dd_add(acc[q], prod);
+          }
         }
+        rhs = dd_neg(dd_add_d(au, d.rd[j]));
+      } else {
+        acc[0] = dd_from(1.0);  // columns that pad the last block: an identity
       }
+      // K(j, j - p): column jr - p of this block's diagonal, or KD + jr - p of the block before
 #pragma unroll
-      for (int p = 0; p <= KD; ++p) st_dd(d.Kh, d.Kl, static_cast<long long>(p) * n + j, acc[p]);
+      for (int p = 0; p <= KD; ++p)
+        if (p <= jr) st_dd(d.Dh, d.Dl, (jr * (jr + 1) / 2 + jr - p) * d.slots + blk, acc[p]);
+        else st_dd(d.Bh, d.Bl, (jr * KD + KD + jr - p) * d.slots + blk, acc[p]);
+      for (int c = 0; c < jr; ++c) st_dd(d.Bh, d.Bl, (jr * KD + c) * d.slots + blk, dd_from(0.0));
+      st_dd(d.Fh, d.Fl, jr * d.slots + blk, rhs);
     }
-    __syncthreads();
-    if (tid == 0) s_bad = 0;
-    __syncthreads();
-    part_factor<KD>(d, &s_bad);
-    if (tid == 0 && s_bad) {
-      d.out->status = SOV_ERROR;
-      d.out->failed = 2;
-      s_stop = 1;
-    }
-    __syncthreads();
-    if (s_stop) break;
+    cluster.sync();
     // ---- predictor (pass 0) and corrector (pass 1) ----
+    double alpha_p = 1.0, alpha_d = 1.0;
+    bool bad = false;
     for (int pass = 0; pass < 2; ++pass) {
-      const double mu = s_mu, sigma = pass ? s_sigma : 0.0;
-      // u = rc / w + theta rp
-      for (int r = tid; r < m; r += kXbThreads) {
-        const double rc = d.w[r] * d.zh[r] + (pass ? d.dwa[r] * d.dza[r] - sigma * mu : 0.0);
-        st_dd(d.uh, d.ul, r, dd_add_d(dd_mul_d(ld_dd(d.rph, d.rpl, r), d.th[r]), rc / d.w[r]));
+      double sigma_mu = 0.0;
+      if (pass == 1) {
+        // mu_aff and sigma = (mu_aff / mu)^3 (qp_interior_point.cpp, as interior_point.cpp:666-673)
+        double ma[1] = {0.0};
+        for (int r = tid; r < m; r += threads) {
+          d.dwa[r] = d.dw[r];
+          d.dza[r] = d.dzh[r];
+          ma[0] += (d.w[r] + alpha_p * d.dw[r]) * (d.zh[r] + alpha_d * d.dzh[r]);
+        }
+        cluster_reduce<1>(ma, ops1, red, cr, turn);
+        const double ratio = (ma[0] / m) / mu;
+        sigma_mu = fmin(1.0, ratio * ratio * ratio) * mu;
+        for (int r = tid; r < m; r += threads) {
+          const double q = (d.w[r] * d.zh[r] + d.dwa[r] * d.dza[r] - sigma_mu) / d.w[r];
+          d.rcw[r] = q;
+          st_dd(d.uh, d.ul, r, dd_add_d(dd_mul_d(ld_dd(d.rph, d.rpl, r), d.th[r]), q));
+        }
+        cluster.sync();
+        for (int j = tid; j < d.size[0] * KD; j += threads) {
+          const int blk = j / KD, jr = j - blk * KD;
+          st_dd(d.Fh, d.Fl, jr * d.slots + blk,
+                j < n ? dd_neg(dd_add_d(col_dot(d, j, d.uh, d.ul), d.rd[j])) : dd_from(0.0));
+        }
+        cluster.sync();
       }
-      __syncthreads();
-      // rhs = -rd - A'u (into dx, solved in place)
-      for (int j = tid; j < n; j += kXbThreads)
-        st_dd(d.dxh, d.dxl, j, dd_neg(dd_add_d(col_dot(d, j, d.uh, d.ul), d.rd[j])));
-      __syncthreads();
-      part_solve<KD>(d, d.dxh, d.dxl);
+      band_newton<KD>(d, pass == 0, tid, threads);
+      if (pass == 0) {
+        bad = *static_cast<volatile int*>(d.bad) != 0;  // every block has its pivots by now
+        if (bad) break;
+      }
       // dw = A dx + rp, dz = -rc / w - theta dw; largest steps to the boundary
       double a[2] = {inf, inf};
-      for (int r = tid; r < m; r += kXbThreads) {
-        const double rc = d.w[r] * d.zh[r] + (pass ? d.dwa[r] * d.dza[r] - sigma * mu : 0.0);
+      for (int r = tid; r < m; r += threads) {
         const dd dwv = dd_add(row_dot(d, r, d.dxh, d.dxl), ld_dd(d.rph, d.rpl, r));
-        const dd dzv = dd_neg(dd_add_d(dd_mul_d(dwv, d.th[r]), rc / d.w[r]));
+        const dd dzv = dd_neg(dd_add_d(dd_mul_d(dwv, d.th[r]), d.rcw[r]));
         d.dw[r] = dwv.hi;
         st_dd(d.dzh, d.dzl, r, dzv);
         if (dwv.hi < 0.0) a[0] = fmin(a[0], -d.w[r] / dwv.hi);
         if (dzv.hi < 0.0) a[1] = fmin(a[1], -d.zh[r] / dzv.hi);
       }
       const int ops2[2] = {2, 2};
-      block_reduce<2>(a, ops2, red);
+      cluster_reduce<2>(a, ops2, red, cr, turn);
+      alpha_p = fmin(1.0, a[0]);
+      alpha_d = fmin(1.0, a[1]);
+    }
+    if (bad) {
       if (tid == 0) {
-        s_alpha_p = fmin(1.0, a[0]);
-        s_alpha_d = fmin(1.0, a[1]);
+        d.out->status = SOV_ERROR;
+        d.out->failed = 2;
       }
-      __syncthreads();
-      if (pass == 0) {
-        // mu_aff and sigma = (mu_aff / mu)^3 (qp_interior_point.cpp, as interior_point.cpp:666-673)
-        const double ap = s_alpha_p, ad = s_alpha_d;
-        double ma[1] = {0.0};
-        for (int r = tid; r < m; r += kXbThreads) {
-          d.dwa[r] = d.dw[r];
-          d.dza[r] = d.dzh[r];
-          ma[0] += (d.w[r] + ap * d.dw[r]) * (d.zh[r] + ad * d.dzh[r]);
-        }
-        block_reduce<1>(ma, ops1, red);
-        if (tid == 0) {
-          const double ratio = (ma[0] / m) / mu;
-          s_sigma = fmin(1.0, ratio * ratio * ratio);
-        }
-        __syncthreads();
-      }
+      break;
     }
     // ---- common step ----
-    const double alpha = fmin(1.0, d.tau * fmin(s_alpha_p, s_alpha_d));
-    for (int j = tid; j < n; j += kXbThreads)
+    const double alpha = fmin(1.0, d.tau * fmin(alpha_p, alpha_d));
+    for (int j = tid; j < n; j += threads)
       st_dd(d.xh, d.xl, j, dd_add(ld_dd(d.xh, d.xl, j), dd_mul_d(ld_dd(d.dxh, d.dxl, j), alpha)));
-    for (int r = tid; r < m; r += kXbThreads) {
+    for (int r = tid; r < m; r += threads) {
       d.w[r] += alpha * d.dw[r];
       st_dd(d.zh, d.zl, r, dd_add(ld_dd(d.zh, d.zl, r), dd_mul_d(ld_dd(d.dzh, d.dzl, r), alpha)));
     }
     if (tid == 0 && it < SOV_HISTORY_MAX) d.out->step_hist[it] = alpha;
-    __syncthreads();
+    cluster.sync();
   }
+  cluster.sync();  // no CTA leaves while another may still write its shared memory
 }
 
 // Starting point: x = -Q^-1 c (the unconstrained minimiser), slack w = Ax - b shifted into the
@@ -700,6 +767,38 @@ __global__ void k_xband_start(XbDev d) {
     d.zh[r] = 1.0 + s_dz;
     d.zl[r] = 0.0;
   }
+}
+
+// One cluster of kXbCluster CTAs (an opt-in size), or of 8 where the device cannot place that one.
+template <int KD>
+void launch_ipm(const XbDev& d, cudaStream_t st) {
+  static int ctas[kMaxDevices] = {};
+  int dev = 0;
+  SOV_CUDA(cudaGetDevice(&dev));
+  if (dev >= kMaxDevices) throw std::runtime_error("double-double QP path: device index beyond the supported 64");
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(kXbThreads);
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  once_per_device(reinterpret_cast<const void*>(k_xband_ipm<KD>), [&] {
+    SOV_CUDA(cudaFuncSetAttribute(k_xband_ipm<KD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    at.val.clusterDim.x = kXbCluster;
+    cfg.gridDim = dim3(kXbCluster);
+    int placed = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&placed, k_xband_ipm<KD>, &cfg);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    ctas[dev] = e == cudaSuccess && placed > 0 ? kXbCluster : 8;
+  });
+  {
+    std::lock_guard<std::mutex> g(once_mutex());  // the write above happened under this lock
+    at.val.clusterDim.x = static_cast<unsigned>(ctas[dev]);
+  }
+  cfg.gridDim = dim3(at.val.clusterDim.x);
+  SOV_CUDA(cudaLaunchKernelEx(&cfg, k_xband_ipm<KD>, d));
 }
 
 template <class T>
@@ -807,16 +906,28 @@ int solve_xband(const sov_model& model, const XBandModel& xb, const sov_options&
   q.put(xb.q);
   c.put(xb.c);
   b.put(xb.b);
-  // n-vectors: xh xl rd dxh dxl; m-vectors: zh zl w th rph rpl uh ul dw dzh dzl dwa dza; band 2 (kd+1) n
-  // segments of the partitioned factorization: one per thread, at least 16 kd columns each
-  int P = std::max(1, std::min(kXbThreads, n / (16 * kd)));
-  if (const char* e = std::getenv("SOVEREIGN_XBAND_SEGMENTS")) P = std::max(1, std::min(P, std::atoi(e)));
-  const size_t nv = 5, mv = 13, kk = static_cast<size_t>(kd) * kd;
-  const size_t part = 2 * (2 * static_cast<size_t>(kd) * n + 3 * P * kk + 2 * P * kk + 2 * static_cast<size_t>(P) * kd);
-  XbBuf<double> work(nv * n + mv * m + 2 * static_cast<size_t>(kd + 1) * n + part, st);
+  // levels of the odd-even reduction over blocks of kd columns
+  XbDev d{};
+  d.size[0] = ceil_div(n, kd);
+  d.off[0] = 0;
+  d.levels = 1;
+  while (d.size[d.levels - 1] > 1) {
+    d.size[d.levels] = (d.size[d.levels - 1] + 1) / 2;
+    d.off[d.levels] = d.off[d.levels - 1] + d.size[d.levels - 1];
+    ++d.levels;
+  }
+  d.slots = d.off[d.levels - 1] + 1;
+  if (const char* e = std::getenv("SOVEREIGN_XBAND_SEGMENTS")) d.natural = std::atoi(e) == 1 ? 1 : 0;
+  // n-vectors: xh xl rd; dx padded to whole blocks: dxh dxl; m-vectors: zh zl w th rph rpl rcw uh ul dw
+  // dzh dzl dwa dza; per block slot: D, L triangles, B X U, F Q I
+  const size_t nv = 3, mv = 14, np = static_cast<size_t>(d.size[0]) * kd;
+  const size_t per_slot = 2 * (static_cast<size_t>(kd) * (kd + 1) / 2 + static_cast<size_t>(kd) * (kd - 1) / 2 +
+                               3 * static_cast<size_t>(kd) * kd + 3 * static_cast<size_t>(kd));
+  XbBuf<double> work(nv * n + 2 * np + mv * m + per_slot * d.slots, st);
+  XbBuf<int> bad(1, st);
+  SOV_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), st));
   XbBuf<XbOut> out(1, st);
   SOV_CUDA(cudaMemsetAsync(out.p, 0, sizeof(XbOut), st));
-  XbDev d{};
   d.n = n;
   d.m = m;
   d.max_iter = std::max(1, opt.max_iterations);
@@ -847,14 +958,15 @@ int solve_xband(const sov_model& model, const XBandModel& xb, const sov_options&
   d.xh = take(n);
   d.xl = take(n);
   d.rd = take(n);
-  d.dxh = take(n);
-  d.dxl = take(n);
+  d.dxh = take(np);
+  d.dxl = take(np);
   d.zh = take(m);
   d.zl = take(m);
   d.w = take(m);
   d.th = take(m);
   d.rph = take(m);
   d.rpl = take(m);
+  d.rcw = take(m);
   d.uh = take(m);
   d.ul = take(m);
   d.dw = take(m);
@@ -862,30 +974,33 @@ int solve_xband(const sov_model& model, const XBandModel& xb, const sov_options&
   d.dzl = take(m);
   d.dwa = take(m);
   d.dza = take(m);
-  d.Kh = take(static_cast<size_t>(kd + 1) * n);
-  d.Kl = take(static_cast<size_t>(kd + 1) * n);
-  d.P = P;
-  d.Wh = take(2 * static_cast<size_t>(kd) * n);
-  d.Wl = take(2 * static_cast<size_t>(kd) * n);
-  d.Ch = take(3 * P * kk);
-  d.Cl = take(3 * P * kk);
-  d.Th = take(2 * P * kk);
-  d.Tl = take(2 * P * kk);
-  d.Rh = take(2 * static_cast<size_t>(P) * kd);
-  d.Rl = take(2 * static_cast<size_t>(P) * kd);
+  const size_t S = static_cast<size_t>(d.slots), tri = static_cast<size_t>(kd) * (kd + 1) / 2, full = static_cast<size_t>(kd) * kd;
+  auto pair = [&](double*& h, double*& l, size_t comps) {
+    h = take(comps * S);
+    l = take(comps * S);
+  };
+  pair(d.Dh, d.Dl, tri);
+  pair(d.Bh, d.Bl, full);
+  pair(d.Fh, d.Fl, kd);
+  pair(d.Lh, d.Ll, tri - kd);
+  pair(d.Ih, d.Il, kd);
+  pair(d.Xh, d.Xl, full);
+  pair(d.Uh, d.Ul, full);
+  pair(d.Qh, d.Ql, kd);
+  d.bad = bad.p;
   d.out = out.p;
   cudaEvent_t e0, e1;
   SOV_CUDA(cudaEventCreate(&e0));
   SOV_CUDA(cudaEventCreate(&e1));
   SOV_CUDA(cudaEventRecord(e0, st));
-  k_xband_start<<<1, kXbThreads, 0, st>>>(d);
-  switch (kd) {
-    case 1: k_xband_ipm<1><<<1, kXbThreads, 0, st>>>(d); break;
-    case 2: k_xband_ipm<2><<<1, kXbThreads, 0, st>>>(d); break;
-    case 3: k_xband_ipm<3><<<1, kXbThreads, 0, st>>>(d); break;
-    default: k_xband_ipm<4><<<1, kXbThreads, 0, st>>>(d); break;
-  }
+  k_xband_start<<<1, 1024, 0, st>>>(d);
   SOV_LAUNCH_CHECK();
+  switch (kd) {
+    case 1: launch_ipm<1>(d, st); break;
+    case 2: launch_ipm<2>(d, st); break;
+    case 3: launch_ipm<3>(d, st); break;
+    default: launch_ipm<4>(d, st); break;
+  }
   SOV_CUDA(cudaEventRecord(e1, st));
   XbOut o;
   std::vector<double> x(n), z(m);
