@@ -43,10 +43,10 @@ namespace cg = cooperative_groups;
 namespace sov {
 namespace {
 
-constexpr int kXbThreads = 256;   // per CTA: a level's step keeps up to seven KD x KD blocks in registers
+constexpr int kXbThreads = 512;   // per CTA
 constexpr int kXbCluster = 16;    // CTAs of the cluster (8, the portable size, where 16 cannot be placed)
 constexpr int kXbMaxLevels = 32;
-constexpr int kXbTop = 512;       // levels of at most this many blocks run in CTA 0 alone
+constexpr int kXbTop = 320;       // levels of at most this many blocks run in CTA 0 alone
 
 struct XbOut {
   int status, iterations, history_len, failed;
@@ -75,8 +75,10 @@ struct XbDev {
   double *Fh, *Fl;  // right-hand sides, kd
   double *Lh, *Ll;  // eliminated blocks: unit lower factor (strict, r (r - 1) / 2 + c),
   double *Ih, *Il;  //   1 / D,
-  double *Xh, *Xl;  //   L^-1 B_o (coupling to the left neighbour), r * kd + c,
-  double *Uh, *Ul;  //   L^-1 B_{o+1}' (coupling to the right neighbour),
+  double *Xh, *Xl;  //   X = L^-1 B_o (coupling to the left neighbour), r * kd + c,
+  double *Uh, *Ul;  //   U = L^-1 B_{o+1}' (coupling to the right neighbour),
+  double *Vh, *Vl;  //   X / D by rows,
+  double *Wh, *Wl;  //   U / D by rows,
   double *Qh, *Ql;  //   L^-1 r_o, kd
   int* bad;         // set on a pivot that is not positive and finite
   XbOut* out;
@@ -99,11 +101,13 @@ __device__ __forceinline__ void st_dd(double* h, double* l, long long i, dd v) {
 // rather than inverted: as stable as the natural order (d.natural = 1, SOVEREIGN_XBAND_SEGMENTS=1,
 // runs that one on one thread). About 14 levels at n = 20002 replace chains of hundreds of
 // dependent double-double steps: what bounds a solve is the latency of one step per level.
-// One thread per even block reads both odd neighbours (the left one's factor is computed twice,
-// which costs less than a barrier between factoring and updating) and stores the right one's.
-// A level takes one cluster barrier until kXbTop blocks are left; the rest runs in CTA 0.
-// Measured (n = 20002, 81 iterations): one CTA with 512 segments and a serial separator chain
-// 300 ms, this form XXX ms.
+// A level is two steps: one thread per odd block factors it and solves for X and U (factor_odd),
+// then one thread per entry of the next level's blocks and right-hand sides forms it from both
+// neighbours (update_even): the arithmetic of a level, about 1100 FP64 instructions per pair of
+// blocks, is spread over all threads and its dependent chain is a few double-double operations.
+// Levels are separated by cluster barriers until kXbTop blocks are left; the rest runs in CTA 0.
+// Measured on the device (n = 20002, 83 iterations): one CTA with 512 segments and a serial
+// separator chain 300 ms; one thread per even block doing a whole level 20.3 ms; this form 17.0 ms.
 template <int KD>
 __device__ __forceinline__ void load_sym(const XbDev& d, long long at, dd (&A)[KD][KD]) {
 #pragma unroll
@@ -171,19 +175,13 @@ __device__ __forceinline__ void lower_solve(const dd (&A)[KD][KD], dd (&v)[KD]) 
     for (int k = 0; k < r; ++k) v[r] = dd_sub(v[r], dd_mul(A[r][k], v[k]));
 }
 
-// D -= M' diag(inv) M (lower triangle), r -= M' diag(inv) q
+// row k of M times inv[k]
 template <int KD>
-__device__ __forceinline__ void even_update(const dd (&M)[KD][KD], const dd (&inv)[KD], const dd (&q)[KD],
-                                            dd (&D)[KD][KD], dd (&r)[KD]) {
+__device__ __forceinline__ void scale_rows(dd (&M)[KD][KD], const dd (&inv)[KD]) {
 #pragma unroll
   for (int k = 0; k < KD; ++k)
 #pragma unroll
-    for (int a = 0; a < KD; ++a) {
-      const dd s = dd_mul(M[k][a], inv[k]);
-#pragma unroll
-      for (int b = 0; b <= a; ++b) D[a][b] = dd_sub(D[a][b], dd_mul(s, M[k][b]));
-      r[a] = dd_sub(r[a], dd_mul(s, q[k]));
-    }
+    for (int c = 0; c < KD; ++c) M[k][c] = dd_mul(M[k][c], inv[k]);
 }
 
 template <int KD>
@@ -197,71 +195,83 @@ __device__ __forceinline__ void store_rhs(double* h, double* l, long long slots,
   for (int k = 0; k < KD; ++k) st_dd(h, l, k * slots + at, v[k]);
 }
 
-// Level l -> l + 1 by `threads` threads from `t`: factor, next level's blocks and right-hand sides.
+// The odd blocks of level l: factor, X and U, q = L^-1 r, one thread per block.
 template <int KD>
-__device__ void reduce_level(const XbDev& d, int l, int t, int threads) {
+__device__ void factor_odd(const XbDev& d, int l, int t, int threads) {
+  const int N = d.size[l];
+  const long long S = d.slots;
+  for (int h = t; h < N / 2; h += threads) {
+    const int i = 2 * h + 1;
+    const long long at = d.off[l] + i;
+    dd A[KD][KD], M[KD][KD], inv[KD], q[KD];
+    load_sym<KD>(d, at, A);
+    load_rhs<KD>(d.Fh, d.Fl, S, at, q);
+    load_full<KD>(d.Bh, d.Bl, S, at, M);
+    if (!block_ldl<KD>(A, inv)) atomicExch(d.bad, 1);
+    store_rhs<KD>(d.Ih, d.Il, S, at, inv);
+#pragma unroll
+    for (int a = 1; a < KD; ++a)
+#pragma unroll
+      for (int b = 0; b < a; ++b) st_dd(d.Lh, d.Ll, (a * (a - 1) / 2 + b) * S + at, A[a][b]);
+    lower_solve<KD>(A, q);
+    store_rhs<KD>(d.Qh, d.Ql, S, at, q);
+    lower_solve<KD>(A, M);
+    store_full<KD>(d.Xh, d.Xl, S, at, M);
+    scale_rows<KD>(M, inv);
+    store_full<KD>(d.Vh, d.Vl, S, at, M);
+    if (i + 1 < N) {
+#pragma unroll
+      for (int a = 0; a < KD; ++a)
+#pragma unroll
+        for (int b = 0; b < KD; ++b) M[a][b] = ld_dd(d.Bh, d.Bl, (b * KD + a) * S + at + 1);
+      lower_solve<KD>(A, M);
+      store_full<KD>(d.Uh, d.Ul, S, at, M);
+      scale_rows<KD>(M, inv);
+      store_full<KD>(d.Wh, d.Wl, S, at, M);
+    }
+  }
+}
+
+// acc -= sum_k P[k][a] Q[k][b] of block `at` (Q a kd x kd block of `ld` columns, or a vector)
+template <int KD>
+__device__ __forceinline__ dd minus_product(dd acc, const double* Ph, const double* Pl, int a, const double* Qh,
+                                            const double* Ql, int ld, int b, long long S, long long at) {
+#pragma unroll
+  for (int k = 0; k < KD; ++k)
+    acc = dd_sub(acc, dd_mul(ld_dd(Ph, Pl, (k * KD + a) * S + at), ld_dd(Qh, Ql, (k * ld + b) * S + at)));
+  return acc;
+}
+
+// Level l + 1 from level l's odd blocks, one thread per entry: D_e (lower triangle), r_e, and the
+// coupling of an even block to the one before it.
+template <int KD>
+__device__ void update_even(const XbDev& d, int l, int t, int threads) {
+  constexpr int kTri = KD * (KD + 1) / 2, kEntries = kTri + KD + KD * KD;
   const int N = d.size[l], Nn = d.size[l + 1];
   const long long S = d.slots, o0 = d.off[l], o1 = d.off[l + 1];
-  for (int h = t; h < Nn; h += threads) {
+  for (int u = t; u < kEntries * Nn; u += threads) {
+    const int entry = u / Nn, h = u - entry * Nn;
     const long long e = o0 + 2 * h;
-    dd D[KD][KD], r[KD], A[KD][KD], M[KD][KD], inv[KD], q[KD];
-    load_sym<KD>(d, e, D);
-    load_rhs<KD>(d.Fh, d.Fl, S, e, r);
-    if (h > 0) {  // left odd block e - 1
-      load_sym<KD>(d, e - 1, A);
-      load_rhs<KD>(d.Fh, d.Fl, S, e - 1, q);
-      dd B[KD][KD], X[KD][KD];
-      load_full<KD>(d.Bh, d.Bl, S, e, B);
-#pragma unroll
-      for (int a = 0; a < KD; ++a)
-#pragma unroll
-        for (int b = 0; b < KD; ++b) M[a][b] = B[b][a];
-      load_full<KD>(d.Bh, d.Bl, S, e - 1, X);
-      block_ldl<KD>(A, inv);
-      lower_solve<KD>(A, M);
-      lower_solve<KD>(A, X);
-      lower_solve<KD>(A, q);
-      even_update<KD>(M, inv, q, D, r);
-#pragma unroll
-      for (int a = 0; a < KD; ++a)
-#pragma unroll
-        for (int b = 0; b < KD; ++b) {
-          dd v = dd_from(0.0);
-#pragma unroll
-          for (int k = 0; k < KD; ++k) v = dd_sub(v, dd_mul(dd_mul(M[k][a], inv[k]), X[k][b]));
-          B[a][b] = v;
-        }
-      store_full<KD>(d.Bh, d.Bl, S, o1 + h, B);
+    const bool left = h > 0, right = 2 * h + 1 < N;
+    if (entry < kTri) {
+      int a = 0;
+      while ((a + 1) * (a + 2) / 2 <= entry) ++a;
+      const int b = entry - a * (a + 1) / 2;
+      dd v = ld_dd(d.Dh, d.Dl, entry * S + e);
+      if (left) v = minus_product<KD>(v, d.Wh, d.Wl, a, d.Uh, d.Ul, KD, b, S, e - 1);
+      if (right) v = minus_product<KD>(v, d.Vh, d.Vl, a, d.Xh, d.Xl, KD, b, S, e + 1);
+      st_dd(d.Dh, d.Dl, entry * S + o1 + h, v);
+    } else if (entry < kTri + KD) {
+      const int a = entry - kTri;
+      dd v = ld_dd(d.Fh, d.Fl, a * S + e);
+      if (left) v = minus_product<KD>(v, d.Wh, d.Wl, a, d.Qh, d.Ql, 1, 0, S, e - 1);
+      if (right) v = minus_product<KD>(v, d.Vh, d.Vl, a, d.Qh, d.Ql, 1, 0, S, e + 1);
+      st_dd(d.Fh, d.Fl, a * S + o1 + h, v);
+    } else if (left) {
+      const int c = entry - kTri - KD, a = c / KD, b = c - a * KD;
+      const dd v = minus_product<KD>(dd_from(0.0), d.Wh, d.Wl, a, d.Xh, d.Xl, KD, b, S, e - 1);
+      st_dd(d.Bh, d.Bl, c * S + o1 + h, v);
     }
-    if (2 * h + 1 < N) {  // right odd block e + 1: its factor is stored here
-      load_sym<KD>(d, e + 1, A);
-      load_rhs<KD>(d.Fh, d.Fl, S, e + 1, q);
-      load_full<KD>(d.Bh, d.Bl, S, e + 1, M);
-      if (!block_ldl<KD>(A, inv)) atomicExch(d.bad, 1);
-      lower_solve<KD>(A, M);
-      lower_solve<KD>(A, q);
-      even_update<KD>(M, inv, q, D, r);
-      store_full<KD>(d.Xh, d.Xl, S, e + 1, M);
-      store_rhs<KD>(d.Ih, d.Il, S, e + 1, inv);
-      store_rhs<KD>(d.Qh, d.Ql, S, e + 1, q);
-#pragma unroll
-      for (int a = 1; a < KD; ++a)
-#pragma unroll
-        for (int b = 0; b < a; ++b) st_dd(d.Lh, d.Ll, (a * (a - 1) / 2 + b) * S + e + 1, A[a][b]);
-      if (2 * h + 2 < N) {
-#pragma unroll
-        for (int a = 0; a < KD; ++a)
-#pragma unroll
-          for (int b = 0; b < KD; ++b) M[a][b] = ld_dd(d.Bh, d.Bl, (b * KD + a) * S + e + 2);
-        lower_solve<KD>(A, M);
-        store_full<KD>(d.Uh, d.Ul, S, e + 1, M);
-      }
-    }
-#pragma unroll
-    for (int a = 0; a < KD; ++a)
-#pragma unroll
-      for (int b = 0; b <= a; ++b) st_dd(d.Dh, d.Dl, (a * (a + 1) / 2 + b) * S + o1 + h, D[a][b]);
-    store_rhs<KD>(d.Fh, d.Fl, S, o1 + h, r);
   }
 }
 
@@ -273,41 +283,32 @@ __device__ __forceinline__ void load_lower(const XbDev& d, long long at, dd (&A)
     for (int b = 0; b < a; ++b) A[a][b] = ld_dd(d.Lh, d.Ll, (a * (a - 1) / 2 + b) * d.slots + at);
 }
 
-// r -= M' diag(inv) q with M, inv of the factored block `at`, from h / l
-template <int KD>
-__device__ __forceinline__ void rhs_update(const XbDev& d, const double* Mh, const double* Ml, long long at,
-                                           const dd (&q)[KD], dd (&r)[KD]) {
-#pragma unroll
-  for (int k = 0; k < KD; ++k) {
-    const dd w = dd_mul(q[k], ld_dd(d.Ih, d.Il, k * d.slots + at));
-#pragma unroll
-    for (int a = 0; a < KD; ++a) r[a] = dd_sub(r[a], dd_mul(ld_dd(Mh, Ml, (k * KD + a) * d.slots + at), w));
-  }
-}
-
-// The right-hand side alone down one level, with the factor reduce_level left.
+// The right-hand side alone down one level, with the factor factor_odd left: one thread per entry
+// (q of the odd neighbours, a few operations, is formed by each of them rather than in a step of its own).
 template <int KD>
 __device__ void forward_level(const XbDev& d, int l, int t, int threads) {
   const int N = d.size[l], Nn = d.size[l + 1];
   const long long S = d.slots, o0 = d.off[l], o1 = d.off[l + 1];
-  for (int h = t; h < Nn; h += threads) {
+  for (int u = t; u < KD * Nn; u += threads) {
+    const int a = u / Nn, h = u - a * Nn;
     const long long e = o0 + 2 * h;
-    dd r[KD], q[KD], A[KD][KD];
-    load_rhs<KD>(d.Fh, d.Fl, S, e, r);
+    dd v = ld_dd(d.Fh, d.Fl, a * S + e), q[KD], A[KD][KD];
     if (h > 0) {
       load_rhs<KD>(d.Fh, d.Fl, S, e - 1, q);
       load_lower<KD>(d, e - 1, A);
       lower_solve<KD>(A, q);
-      rhs_update<KD>(d, d.Uh, d.Ul, e - 1, q, r);
+#pragma unroll
+      for (int k = 0; k < KD; ++k) v = dd_sub(v, dd_mul(ld_dd(d.Wh, d.Wl, (k * KD + a) * S + e - 1), q[k]));
     }
     if (2 * h + 1 < N) {
       load_rhs<KD>(d.Fh, d.Fl, S, e + 1, q);
       load_lower<KD>(d, e + 1, A);
       lower_solve<KD>(A, q);
-      rhs_update<KD>(d, d.Xh, d.Xl, e + 1, q, r);
-      store_rhs<KD>(d.Qh, d.Ql, S, e + 1, q);
+#pragma unroll
+      for (int k = 0; k < KD; ++k) v = dd_sub(v, dd_mul(ld_dd(d.Vh, d.Vl, (k * KD + a) * S + e + 1), q[k]));
+      if (a == 0) store_rhs<KD>(d.Qh, d.Ql, S, e + 1, q);
     }
-    store_rhs<KD>(d.Fh, d.Fl, S, o1 + h, r);
+    st_dd(d.Fh, d.Fl, a * S + o1 + h, v);
   }
 }
 
@@ -323,38 +324,43 @@ __device__ __forceinline__ void upper_solve(const dd (&A)[KD][KD], const dd (&in
 }
 
 // The odd blocks of level l from their even neighbours; block i of level l is block i << l of the
-// matrix, and solutions go straight to their place in dx.
+// matrix, and solutions go straight to their place in dx. A group of lanes takes a block: lane k
+// forms entry k of q - X x_left - U x_right, then all lanes of the group run the small L' solve.
 template <int KD>
 __device__ void backward_level(const XbDev& d, int l, int t, int threads) {
+  constexpr int kLanes = KD <= 2 ? KD : 4;
   const int N = d.size[l], odd = N / 2;
   const long long S = d.slots, o0 = d.off[l];
-  for (int h = t; h < odd; h += threads) {
-    const int i = 2 * h + 1;
+  const int lane = t % kLanes, k = lane < KD ? lane : KD - 1;
+  // whole warps stay in the loop together: the group exchanges its entries by shuffles
+  const int warp0 = t & ~31;
+  for (int base = warp0 / kLanes; base < odd; base += threads / kLanes) {
+    const int h = base + (t - warp0) / kLanes;
+    const int i = 2 * min(h, odd - 1) + 1;
     const long long at = o0 + i;
-    dd v[KD], inv[KD], A[KD][KD];
-    load_rhs<KD>(d.Qh, d.Ql, S, at, v);
-    load_rhs<KD>(d.Ih, d.Il, S, at, inv);
-    load_lower<KD>(d, at, A);
+    dd v = ld_dd(d.Qh, d.Ql, k * S + at);
     const long long c0 = static_cast<long long>(i - 1) * KD << l;
 #pragma unroll
-    for (int c = 0; c < KD; ++c) {
-      const dd x = ld_dd(d.dxh, d.dxl, c0 + c);
-#pragma unroll
-      for (int k = 0; k < KD; ++k) v[k] = dd_sub(v[k], dd_mul(ld_dd(d.Xh, d.Xl, (k * KD + c) * S + at), x));
-    }
+    for (int c = 0; c < KD; ++c) v = dd_sub(v, dd_mul(ld_dd(d.Xh, d.Xl, (k * KD + c) * S + at), ld_dd(d.dxh, d.dxl, c0 + c)));
     if (i + 1 < N) {
       const long long c1 = static_cast<long long>(i + 1) * KD << l;
 #pragma unroll
-      for (int c = 0; c < KD; ++c) {
-        const dd x = ld_dd(d.dxh, d.dxl, c1 + c);
-#pragma unroll
-        for (int k = 0; k < KD; ++k) v[k] = dd_sub(v[k], dd_mul(ld_dd(d.Uh, d.Ul, (k * KD + c) * S + at), x));
-      }
+      for (int c = 0; c < KD; ++c) v = dd_sub(v, dd_mul(ld_dd(d.Uh, d.Ul, (k * KD + c) * S + at), ld_dd(d.dxh, d.dxl, c1 + c)));
     }
-    upper_solve<KD>(A, inv, v);
-    const long long ci = static_cast<long long>(i) * KD << l;
+    dd x[KD], inv[KD], A[KD][KD];
 #pragma unroll
-    for (int k = 0; k < KD; ++k) st_dd(d.dxh, d.dxl, ci + k, v[k]);
+    for (int j = 0; j < KD; ++j) {
+      x[j].hi = __shfl_sync(kFull, v.hi, j, kLanes);
+      x[j].lo = __shfl_sync(kFull, v.lo, j, kLanes);
+    }
+    load_rhs<KD>(d.Ih, d.Il, S, at, inv);
+    load_lower<KD>(d, at, A);
+    upper_solve<KD>(A, inv, x);
+    if (h < odd && lane == 0) {
+      const long long ci = static_cast<long long>(i) * KD << l;
+#pragma unroll
+      for (int j = 0; j < KD; ++j) st_dd(d.dxh, d.dxl, ci + j, x[j]);
+    }
   }
 }
 
@@ -419,11 +425,21 @@ __device__ void solve_natural(const XbDev& d, bool factor) {
 #pragma unroll
         for (int b = 0; b < KD; ++b) M[a][b] = ld_dd(d.Bh, d.Bl, (b * KD + a) * S + i + 1);
       lower_solve<KD>(A, M);
-      even_update<KD>(M, inv, q, D, r);
       store_full<KD>(d.Uh, d.Ul, S, i, M);
-    } else {
-      rhs_update<KD>(d, d.Uh, d.Ul, i, q, r);
+#pragma unroll
+      for (int k = 0; k < KD; ++k)
+#pragma unroll
+        for (int a = 0; a < KD; ++a) {
+          const dd w = dd_mul(M[k][a], inv[k]);
+#pragma unroll
+          for (int b = 0; b <= a; ++b) D[a][b] = dd_sub(D[a][b], dd_mul(w, M[k][b]));
+          st_dd(d.Wh, d.Wl, (k * KD + a) * S + i, w);
+        }
     }
+#pragma unroll
+    for (int a = 0; a < KD; ++a)
+#pragma unroll
+      for (int k = 0; k < KD; ++k) r[a] = dd_sub(r[a], dd_mul(ld_dd(d.Wh, d.Wl, (k * KD + a) * S + i), q[k]));
   }
   dd x[KD];
   for (int i = N - 1; i >= 0; --i) {
@@ -458,16 +474,26 @@ __device__ void band_newton(const XbDev& d, bool factor, int t, int threads) {
   }
   int l = 0;
   for (; d.size[l] > kXbTop; ++l) {
-    if (factor) reduce_level<KD>(d, l, t, threads);
-    else forward_level<KD>(d, l, t, threads);
+    if (factor) {
+      factor_odd<KD>(d, l, t, threads);
+      cluster.sync();
+      update_even<KD>(d, l, t, threads);
+    } else {
+      forward_level<KD>(d, l, t, threads);
+    }
     cluster.sync();
   }
   if (cluster.block_rank() == 0) {
     const int tt = threadIdx.x;
     int u = l;
     for (; u + 1 < d.levels; ++u) {
-      if (factor) reduce_level<KD>(d, u, tt, kXbThreads);
-      else forward_level<KD>(d, u, tt, kXbThreads);
+      if (factor) {
+        factor_odd<KD>(d, u, tt, kXbThreads);
+        __syncthreads();
+        update_even<KD>(d, u, tt, kXbThreads);
+      } else {
+        forward_level<KD>(d, u, tt, kXbThreads);
+      }
       __syncthreads();
     }
     if (tt == 0) solve_last<KD>(d, factor);
@@ -502,7 +528,7 @@ __device__ __forceinline__ dd col_dot(const XbDev& d, int j, const double* uh, c
 // all CTAs' shared memory, and after one cluster barrier every thread folds them in rank order.
 // Two buffers taken in turn: a buffer is written again only after a later barrier.
 struct ClusterRed {
-  double v[2][4][kXbCluster];
+  double v[2][5][kXbCluster];
 };
 template <int NV>
 __device__ __forceinline__ void cluster_reduce(double (&v)[NV], const int (&ops)[NV], double* red, ClusterRed& cr,
@@ -534,12 +560,14 @@ __device__ __forceinline__ void cluster_reduce(double (&v)[NV], const int (&ops)
 
 template <int KD>
 __global__ void __launch_bounds__(kXbThreads, 1) k_xband_ipm(const __grid_constant__ XbDev d) {
-  __shared__ double red[4 * 32];
+  __shared__ double red[5 * 32];
   __shared__ ClusterRed cr;
   cg::cluster_group cluster = cg::this_cluster();
   int turn = 0;
   const int threads = static_cast<int>(cluster.num_blocks()) * kXbThreads;
-  const int tid = static_cast<int>(cluster.block_rank()) * kXbThreads + static_cast<int>(threadIdx.x);
+  // warps numbered across the CTAs, so that a level with fewer blocks than threads uses every SM
+  const int tid = static_cast<int>((threadIdx.x >> 5) * cluster.num_blocks() + cluster.block_rank()) * 32 +
+                  static_cast<int>(threadIdx.x & 31);
   const int n = d.n, m = d.m;
   const double inf = INFINITY;
   // the reference QP stops at its tolerances; this path goes two decades further (cheap in
@@ -550,7 +578,7 @@ __global__ void __launch_bounds__(kXbThreads, 1) k_xband_ipm(const __grid_consta
   int it = 0;
   for (;; ++it) {
     // ---- residuals, mu, objective; theta and the predictor's u = rc / w + theta rp ----
-    double v[4] = {0.0, 0.0, 0.0, 0.0};  // max |rp|, max |rd|, max |Qx|, w'z
+    double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // max |rp|, max |rd|, max |Qx|, w'z, objective
     for (int r = tid; r < m; r += threads) {
       const double w = d.w[r], z = d.zh[r], th = z / w;
       const dd rp = dd_add_d(dd_add_d(row_dot(d, r, d.xh, d.xl), -w), -d.b[r]);
@@ -564,23 +592,19 @@ __global__ void __launch_bounds__(kXbThreads, 1) k_xband_ipm(const __grid_consta
       v[0] = fmax(v[0], fabs(rp.hi));
       v[3] += w * z;
     }
-    double objp = 0.0;
     for (int j = tid; j < n; j += threads) {
       const dd qx = dd_mul_d(ld_dd(d.xh, d.xl, j), d.q[j]);
       const dd rd = dd_sub(dd_add_d(qx, d.c[j]), col_dot(d, j, d.zh, d.zl));
       d.rd[j] = rd.hi;
       v[1] = fmax(v[1], fabs(rd.hi));
       v[2] = fmax(v[2], fabs(qx.hi));
-      objp += d.c[j] * d.xh[j] + 0.5 * d.q[j] * d.xh[j] * d.xh[j];
+      v[4] += d.c[j] * d.xh[j] + 0.5 * d.q[j] * d.xh[j] * d.xh[j];
     }
-    const int ops4[4] = {1, 1, 1, 0};
-    cluster_reduce<4>(v, ops4, red, cr, turn);
-    double o1[1] = {objp};
-    const int ops1[1] = {0};
-    cluster_reduce<1>(o1, ops1, red, cr, turn);
+    const int ops5[5] = {1, 1, 1, 0, 0}, ops1[1] = {0};
+    cluster_reduce<5>(v, ops5, red, cr, turn);
     // every thread holds the same sums, so the whole cluster takes the same decision
     const double mu = v[3] / m;
-    const double obj = o1[0] + d.obj_constant;
+    const double obj = v[4] + d.obj_constant;
     const double p_res = v[0] / d.bnorm;
     const double d_res = v[1] / fmax(1.0, d.cnorm + v[2]);
     const double gap = v[3] / (1.0 + fabs(obj));
@@ -919,10 +943,10 @@ int solve_xband(const sov_model& model, const XBandModel& xb, const sov_options&
   d.slots = d.off[d.levels - 1] + 1;
   if (const char* e = std::getenv("SOVEREIGN_XBAND_SEGMENTS")) d.natural = std::atoi(e) == 1 ? 1 : 0;
   // n-vectors: xh xl rd; dx padded to whole blocks: dxh dxl; m-vectors: zh zl w th rph rpl rcw uh ul dw
-  // dzh dzl dwa dza; per block slot: D, L triangles, B X U, F Q I
+  // dzh dzl dwa dza; per block slot: D, L triangles, B X U V W, F Q I
   const size_t nv = 3, mv = 14, np = static_cast<size_t>(d.size[0]) * kd;
   const size_t per_slot = 2 * (static_cast<size_t>(kd) * (kd + 1) / 2 + static_cast<size_t>(kd) * (kd - 1) / 2 +
-                               3 * static_cast<size_t>(kd) * kd + 3 * static_cast<size_t>(kd));
+                               5 * static_cast<size_t>(kd) * kd + 3 * static_cast<size_t>(kd));
   XbBuf<double> work(nv * n + 2 * np + mv * m + per_slot * d.slots, st);
   XbBuf<int> bad(1, st);
   SOV_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), st));
@@ -986,6 +1010,8 @@ int solve_xband(const sov_model& model, const XBandModel& xb, const sov_options&
   pair(d.Ih, d.Il, kd);
   pair(d.Xh, d.Xl, full);
   pair(d.Uh, d.Ul, full);
+  pair(d.Vh, d.Vl, full);
+  pair(d.Wh, d.Wl, full);
   pair(d.Qh, d.Ql, kd);
   d.bad = bad.p;
   d.out = out.p;
