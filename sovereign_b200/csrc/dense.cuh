@@ -70,6 +70,12 @@ template <class T>
 void dense_solve(const DenseSystem<T>& s, double* z, unsigned& epoch, int* err, cudaStream_t st,
                  int* launches);
 
+// Y <- L^-1 Y for nrhs columns (column-major, ldy >= mp, padding rows 0). `flags`: dense_forward_flags
+// entries of device memory, cleared by the call; *err is set if a wait gives up.
+size_t dense_forward_flags(int nb, int nrhs);
+void dense_forward_multi(const DenseSystem<double>& s, double* Y, int ldy, int nrhs, unsigned* flags, int* err,
+                         cudaStream_t st, int* launches);
+
 // Number of CTAs the dataflow solve may use (all co-resident).
 int dataflow_grid(int nb);
 

@@ -301,12 +301,12 @@ class Engine {
   static constexpr int kLongRow = 512;
   DevBuf<double> sigma_, tr_, dyv_;
   // QP with a coupled Hessian: dense H = Q + diag(h) (order n, padded to nph_), its factor, and
-  // Y = H^-1 A' for the reduced system M = A H^-1 A'
+  // Y = L^-1 A' (H = L L') for the reduced system M = A H^-1 A' = Y'Y
   bool coupled_ = false;
   int nph_ = 0, nbh_ = 0;
   DevBuf<int> q_ptr_, q_idx_;
   DevBuf<double> q_val_, qdense_, hmat_, hlinv_, hdiag_, ymat_, hvec_;
-  DevBuf<unsigned> hflags_;
+  DevBuf<unsigned> hflags_, hfwd_flags_;
   DenseSystem<double> dsh_{};
   void coupled_newton(int mode);
   // QP second attempt: Mehrotra's starting point in place of the default one
@@ -486,6 +486,7 @@ void Engine::setup() {
     hflags_.alloc(nbh_ + 1);
     hflags_.zero(st_);
     ymat_.alloc(static_cast<size_t>(nph_) * std::max(1, m));
+    hfwd_flags_.alloc(dense_forward_flags(nbh_, m));
     hvec_.alloc(nph_);
     hvec_.zero(st_);
   }
@@ -646,16 +647,15 @@ void Engine::assemble_and_factor(int mode) {
       ds64_ = DenseSystem<double>{M64_.p, Linv64_.p, diag_.p, order_, mp_, nb_, &sc_.p->drops, &sc_.p->fail, flags_.p, flags_.p + nb_, 1e-13};
     }
     if (coupled_ && mode != kWeightOnes) {
-      // H = Q + diag(h), factored; Y = H^-1 A'; M = A Y + reg I, factored (the starting-point
-      // system has H = I and takes the ordinary assembly below)
+      // H = Q + diag(h) = L L'; Y = L^-1 A'; M = A H^-1 A' + reg I = Y'Y + reg I, factored (the
+      // starting-point system has H = I and takes the ordinary assembly below)
       SOV_CUDA(cudaMemcpyAsync(hmat_.p, qdense_.p, sizeof(double) * static_cast<size_t>(nph_) * nph_,
                                cudaMemcpyDeviceToDevice, st_));
       launch_hessian_diag(dev_, false, hmat_.p, nph_, hdiag_.p, st_);
       dense_cholesky<double>(dsh_, st_, &launches_);
       SOV_CUDA(cudaMemsetAsync(ymat_.p, 0, sizeof(double) * static_cast<size_t>(nph_) * std::max(1, f_.m), st_));
       launch_rows_to_columns(dev_, ymat_.p, nph_, st_);
-      for (int i = 0; i < f_.m; ++i)
-        dense_solve<double>(dsh_, ymat_.p + static_cast<size_t>(i) * nph_, epoch_, err_.p, st_, &launches_);
+      dense_forward_multi(dsh_, ymat_.p, nph_, f_.m, hfwd_flags_.p, err_.p, st_, &launches_);
       launch_dense_clear<double>(M64_.p, order_, mp_, st_);
       launch_form_normal(dev_, ymat_.p, nph_, M64_.p, mp_, reg, diag_.p, st_);
       dense_cholesky<double>(ds64_, st_, &launches_);

@@ -568,26 +568,49 @@ __global__ void __launch_bounds__(kThreads) k_rows_to_columns(IpmDev d, double* 
       Y[static_cast<int64_t>(i) * ld + d.col_idx[p]] = d.rval[p];
 }
 
-// one warp per lower-triangle entry (i, k), k <= i: sum over row i of A of a_ij Y[j][k]
+// Lower triangle of M = Y'Y: a warp per 4 x 4 block of entries, its lanes along the columns of Y (8
+// coalesced loads for 16 products; with a warp per entry every column was read again for every row)
 __global__ void __launch_bounds__(kThreads) k_form_normal(IpmDev d, const double* Y, int ld_y, double* M, int ld_m,
                                                           double reg, double* diag) {
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * (blockDim.x >> 5);
-  const int64_t pairs = static_cast<int64_t>(d.m) * (d.m + 1) / 2;
-  for (int64_t t = warp_row(); t < pairs; t += warps) {
-    int i = static_cast<int>((sqrt(8.0 * static_cast<double>(t) + 1.0) - 1.0) * 0.5);
-    while (static_cast<int64_t>(i + 1) * (i + 2) / 2 <= t) ++i;
-    while (static_cast<int64_t>(i) * (i + 1) / 2 > t) --i;
-    const int k = static_cast<int>(t - static_cast<int64_t>(i) * (i + 1) / 2);
-    const double* yk = Y + static_cast<int64_t>(k) * ld_y;
-    double acc = 0.0;
-    for (int p = d.row_ptr[i] + lane; p < d.row_ptr[i + 1]; p += 32) acc += d.rval[p] * yk[d.col_idx[p]];
-    acc = warp_sum(acc);
-    if (lane == 0) {
-      const double v = i == k ? acc + reg : acc;
-      M[static_cast<int64_t>(k) * ld_m + i] = v;
-      if (i == k) diag[i] = v;
+  const int mt = (d.m + 3) / 4;
+  const int64_t tiles = static_cast<int64_t>(mt) * (mt + 1) / 2;
+  for (int64_t t = warp_row(); t < tiles; t += warps) {
+    int ti = static_cast<int>((sqrt(8.0 * static_cast<double>(t) + 1.0) - 1.0) * 0.5);
+    while (static_cast<int64_t>(ti + 1) * (ti + 2) / 2 <= t) ++ti;
+    while (static_cast<int64_t>(ti) * (ti + 1) / 2 > t) --ti;
+    const int tk = static_cast<int>(t - static_cast<int64_t>(ti) * (ti + 1) / 2);
+    const double *yi[4], *yk[4];  // columns past m are clamped to the last one, their entries not stored
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      yi[q] = Y + static_cast<int64_t>(min(4 * ti + q, d.m - 1)) * ld_y;
+      yk[q] = Y + static_cast<int64_t>(min(4 * tk + q, d.m - 1)) * ld_y;
     }
+    double acc[4][4] = {};
+    for (int j = lane; j < d.n; j += 32) {
+      double vi[4], vk[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        vi[q] = yi[q][j];
+        vk[q] = yk[q][j];
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[q][r] += vi[q] * vk[r];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const double v0 = warp_sum(acc[q][r]);
+        const int i = 4 * ti + q, k = 4 * tk + r;
+        if (lane != 0 || i >= d.m || k > i) continue;
+        const double v = i == k ? v0 + reg : v0;
+        M[static_cast<int64_t>(k) * ld_m + i] = v;
+        if (i == k) diag[i] = v;
+      }
   }
 }
 
@@ -762,8 +785,8 @@ void launch_rows_to_columns(const IpmDev& d, double* Y, int ld, cudaStream_t st)
 
 void launch_form_normal(const IpmDev& d, const double* Y, int ld_y, double* M, int ld_m, double reg, double* diag,
                         cudaStream_t st) {
-  const long long pairs = static_cast<long long>(d.m) * (d.m + 1) / 2;
-  k_form_normal<<<std::max(1, std::min(kMaxBlocks, ceil_div(pairs * 32, kThreads))), kThreads, 0, st>>>(
+  const long long mt = (d.m + 3) / 4, tiles = mt * (mt + 1) / 2;
+  k_form_normal<<<std::max(1, std::min(kMaxBlocks, ceil_div(tiles * 32, kThreads))), kThreads, 0, st>>>(
       d, Y, ld_y, M, ld_m, reg, diag);
   SOV_LAUNCH_CHECK();
 }

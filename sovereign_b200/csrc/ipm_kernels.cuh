@@ -109,7 +109,7 @@ void launch_xspace_diag(const IpmDev& d, int mode, double* M, int layout_ld, dou
 void launch_hessian_diag(const IpmDev& d, bool start, double* H, int ld, double* diag, cudaStream_t st);
 // Y[:, i] = row i of A (Y zeroed by the caller, column-major, ld)
 void launch_rows_to_columns(const IpmDev& d, double* Y, int ld, cudaStream_t st);
-// lower triangle of M = A Y (Y = H^-1 A', ld_y), reg added on the diagonal; diag[i] = M_ii
+// lower triangle of M = Y'Y (Y = L^-1 A' with H = L L', ld_y), reg added on the diagonal; diag[i] = M_ii
 void launch_form_normal(const IpmDev& d, const double* Y, int ld_y, double* M, int ld_m, double reg, double* diag,
                         cudaStream_t st);
 // r1 of the current mode into v (entries n.. untouched)
