@@ -16,6 +16,21 @@ namespace sov {
 namespace {
 
 constexpr int kSparseThreads = 256;
+constexpr int kCtaThreads = 1024;  // the one-CTA forms
+
+// Threads of a walk over the levels and the barrier between them: the whole grid, or one CTA.
+struct GridWalk {
+  cg::grid_group g;
+  __device__ GridWalk() : g(cg::this_grid()) {}
+  __device__ int rank() const { return static_cast<int>(g.thread_rank()); }
+  __device__ int size() const { return static_cast<int>(g.size()); }
+  __device__ void sync() const { g.sync(); }
+};
+struct CtaWalk {
+  __device__ int rank() const { return static_cast<int>(threadIdx.x); }
+  __device__ int size() const { return static_cast<int>(blockDim.x); }
+  __device__ void sync() const { __syncthreads(); }
+};
 
 __device__ __forceinline__ double warp_total(double v) {
 #pragma unroll
@@ -26,9 +41,12 @@ __device__ __forceinline__ double warp_total(double v) {
 // Per level: the pivots of its columns (one thread each), then its rank-1 updates, one warp per
 // piece: lane l sums the piece's terms l, l + 32, ... and the warp adds the 32 partial sums in a
 // fixed tree; a run cut into pieces is finished by its combine step (deterministic either way).
-__global__ void __launch_bounds__(kSparseThreads) k_sparse_factor(SparseDev s) {
-  cg::grid_group g = cg::this_grid();
-  const int rank = static_cast<int>(g.thread_rank()), size = static_cast<int>(g.size());
+// After the last level the rows of L are left scaled for the one-CTA forward solve (fval = L~ / D by
+// rows; the grid form gains nothing from it).
+template <class Walk>
+__device__ __forceinline__ void factor_levels(const SparseDev& s) {
+  const Walk g;
+  const int rank = g.rank(), size = g.size();
   const int lane = threadIdx.x & 31, warp = rank >> 5, warps = size >> 5;
   int drops = 0, bad = 0;
   for (int h = 0; h < s.levels; ++h) {
@@ -72,9 +90,13 @@ __global__ void __launch_bounds__(kSparseThreads) k_sparse_factor(SparseDev s) {
     }
     g.sync();
   }
+  for (int t = rank; s.fval && t < s.nnz; t += size) s.fval[t] = s.V[s.m + s.row_pos[t]] * s.inv_d[s.row_col[t]];
   if (drops) atomicAdd(s.drop_count, drops);
   if (bad) atomicExch(s.fail, 1);
 }
+
+__global__ void __launch_bounds__(kSparseThreads) k_sparse_factor(SparseDev s) { factor_levels<GridWalk>(s); }
+__global__ void __launch_bounds__(kCtaThreads, 1) k_sparse_factor_cta(SparseDev s) { factor_levels<CtaWalk>(s); }
 
 // L D L' x = z: forward y_k = z_k - sum_j L~_kj (1/D_j) y_j (row k of L, descendants: earlier
 // levels), backward x_k = (1/D_k) (y_k - sum_i L~_ik x_i) (column k, ancestors: later levels);
@@ -149,6 +171,119 @@ __global__ void __launch_bounds__(kSparseThreads) k_sparse_solve(SparseDev s, do
   for (int k = rank; k < s.m; k += size) z[s.perm[k]] = s.work[k];
 }
 
+// The same solve on one CTA with the right-hand side in shared memory: a barrier between levels is
+// a CTA barrier and a gather of it costs tens of cycles, where the grid form pays a grid barrier and
+// dependent L2 loads per level (4.4 us a level each way). The pieces of level h + 2 and the terms of
+// level h + 1 are loaded while level h is summed, so only shared-memory accesses sit between two
+// barriers. Same pieces, same order of every sum: bit-identical to the grid form.
+constexpr int kAhead = 4;  // terms of a short piece loaded a level ahead
+
+template <bool kForward>
+__device__ __forceinline__ void sweep_levels(const SparseDev& s, double* work, const int* piece_lvl, const int* warp_lvl,
+                                             const int* comb_lvl) {
+  const int4* pieces = kForward ? s.lpiece : s.upiece;
+  const int4* combs = kForward ? s.lcomb : s.ucomb;
+  const double* vals = kForward ? s.fval : s.V + s.m;
+  const int* idx = kForward ? s.row_col : s.li;
+  const int tid = static_cast<int>(threadIdx.x), lane = tid & 31, warp = tid >> 5;
+  const int levels = s.levels;
+  auto level = [&](int q) { return kForward ? q : levels - 1 - q; };
+  auto load_piece = [&](int q) {  // this thread's first short piece of the q-th level walked
+    if (q < levels) {
+      const int h = level(q), at = piece_lvl[h] + tid;
+      if (at < warp_lvl[h]) return pieces[at];
+    }
+    return make_int4(0, 0, -1, -1);
+  };
+  struct Terms {
+    double v[kAhead], inv;
+    int c[kAhead];
+  };
+  auto load_terms = [&](const int4& pc, Terms& t) {
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const bool on = pc.x + u < pc.y;
+      t.v[u] = on ? vals[pc.x + u] : 0.0;
+      t.c[u] = on ? idx[pc.x + u] : 0;
+    }
+    t.inv = !kForward && pc.z >= 0 && pc.w < 0 ? s.inv_d[pc.z] : 0.0;
+  };
+  auto apply = [&](const int4& pc, double acc, double inv) {
+    if (pc.w >= 0) s.partial[pc.w] = acc;
+    else if (kForward) work[pc.z] -= acc;
+    else work[pc.z] = (work[pc.z] - acc) * inv;
+  };
+  int4 pc = load_piece(0), pn = load_piece(1);
+  Terms tc, tn;
+  load_terms(pc, tc);
+  for (int q = 0; q < levels; ++q) {
+    const int h = level(q);
+    const int4 pf = load_piece(q + 2);
+    load_terms(pn, tn);
+    if (pc.z >= 0) {
+      double acc = 0.0;
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if (pc.x + u < pc.y) acc += tc.v[u] * work[tc.c[u]];
+      for (int t = pc.x + kAhead; t < pc.y; ++t) acc += vals[t] * work[idx[t]];
+      apply(pc, acc, tc.inv);
+    }
+    for (int at = piece_lvl[h] + tid + kCtaThreads; at < warp_lvl[h]; at += kCtaThreads) {
+      const int4 p2 = pieces[at];
+      double acc = 0.0;
+      for (int t = p2.x; t < p2.y; ++t) acc += vals[t] * work[idx[t]];
+      apply(p2, acc, kForward || p2.w >= 0 ? 0.0 : s.inv_d[p2.z]);
+    }
+    for (int at = warp_lvl[h] + warp; at < piece_lvl[h + 1]; at += kCtaThreads / 32) {
+      const int4 p2 = pieces[at];
+      double acc = 0.0;
+      for (int t = p2.x + lane; t < p2.y; t += 32) acc += vals[t] * work[idx[t]];
+      acc = warp_total(acc);
+      if (lane == 0) apply(p2, acc, kForward || p2.w >= 0 ? 0.0 : s.inv_d[p2.z]);
+    }
+    if (comb_lvl[h + 1] > comb_lvl[h]) {  // uniform: every thread reads the same bounds
+      __syncthreads();
+      for (int c = comb_lvl[h] + tid; c < comb_lvl[h + 1]; c += kCtaThreads) {
+        const int4 cb = combs[c];
+        double t = 0.0;
+        for (int k = 0; k < cb.z; ++k) t += s.partial[cb.y + k];
+        if (kForward) work[cb.x] -= t;
+        else work[cb.x] = (work[cb.x] - t) * s.inv_d[cb.x];
+      }
+    }
+    __syncthreads();
+    pc = pn;
+    pn = pf;
+    tc = tn;
+  }
+}
+
+// work (m doubles) | six level arrays (levels + 1 ints each)
+size_t cta_solve_smem(int m, int levels) {
+  return sizeof(double) * static_cast<size_t>(m) + sizeof(int) * 6 * (static_cast<size_t>(levels) + 1);
+}
+
+__global__ void __launch_bounds__(kCtaThreads, 1) k_sparse_solve_cta(SparseDev s, double* z, const int* run) {
+  if (run && !*run) return;
+  extern __shared__ double sm[];
+  double* work = sm;
+  int* lv = reinterpret_cast<int*>(sm + s.m);
+  const int L1 = s.levels + 1, tid = static_cast<int>(threadIdx.x);
+  for (int h = tid; h < L1; h += kCtaThreads) {
+    lv[h] = s.lpiece_lvl[h];
+    lv[L1 + h] = h < s.levels ? s.lwarp_lvl[h] : 0;
+    lv[2 * L1 + h] = s.lcomb_lvl[h];
+    lv[3 * L1 + h] = s.upiece_lvl[h];
+    lv[4 * L1 + h] = h < s.levels ? s.uwarp_lvl[h] : 0;
+    lv[5 * L1 + h] = s.ucomb_lvl[h];
+  }
+  for (int k = tid; k < s.m; k += kCtaThreads) work[k] = z[s.perm[k]];
+  __syncthreads();
+  sweep_levels<true>(s, work, lv, lv + L1, lv + 2 * L1);
+  sweep_levels<false>(s, work, lv + 3 * L1, lv + 4 * L1, lv + 5 * L1);
+  for (int k = tid; k < s.m; k += kCtaThreads) z[s.perm[k]] = work[k];
+}
+
 template <class T>
 T* put(std::vector<void*>& bufs, const std::vector<T>& h, cudaStream_t st) {
   T* p = nullptr;
@@ -171,6 +306,7 @@ void SparseFactor::upload(const SparseSymbolic& s, int* drop_count, int* fail, d
   d_.V = put(bufs_, std::vector<double>(m + s.li.size(), 0.0), st);
   d_.diag = put(bufs_, std::vector<double>(m, 0.0), st);
   d_.inv_d = put(bufs_, std::vector<double>(m, 0.0), st);
+  d_.nnz = static_cast<int>(s.li.size());
   d_.work = put(bufs_, std::vector<double>(m, 0.0), st);
   d_.perm = put(bufs_, s.perm, st);
   d_.lp = put(bufs_, s.lp, st);
@@ -219,6 +355,24 @@ void SparseFactor::upload(const SparseSymbolic& s, int* drop_count, int* fail, d
   SOV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, k_sparse_solve, kSparseThreads, 0));
   // one CTA per SM: most levels hold few columns, and a grid barrier costs more with more CTAs
   grid_ = std::max(1, sms * std::min(1, std::min(per_sm, per_sm2)));
+  // One CTA where the levels' barriers outweigh what one SM streams. Grid form: 4.2 us a barrier,
+  // two barriers a level. One CTA, measured: solve 1.3 us a level and sweep, plus about 2 ns an
+  // entry of L, and its right-hand side has to fit in shared memory; factor 2 us a level plus about
+  // 4 ns an update term. Solve / factor, grid -> one CTA: chain QP of KKT order 16251 (64 levels,
+  // nnz(L) 44059) 564 -> 232 / 539 -> 465 us; order 26001 (70 levels, nnz(L) 70585) 616 -> 463 us /
+  // 590 against 666 us, so its factor stays on the grid; 60 x 60 grid LP (212 levels) 1.9 -> 0.94 ms.
+  int smem_max = 0;
+  SOV_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  const size_t smem = cta_solve_smem(m, levels);
+  cta_factor_ = static_cast<long long>(S.up_col.size()) <= 1600LL * levels;
+  cta_solve_ = smem <= static_cast<size_t>(smem_max) && nnz_l_ <= 3000LL * levels;
+  if (cta_solve_) {
+    d_.fval = put(bufs_, std::vector<double>(s.li.size(), 0.0), st);
+    SOV_CUDA(cudaStreamSynchronize(st));
+    once_per_device((const void*)k_sparse_solve_cta, [&] {
+      SOV_CUDA(cudaFuncSetAttribute(k_sparse_solve_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
+    });
+  }
 }
 
 void SparseFactor::release() {
@@ -229,16 +383,26 @@ void SparseFactor::release() {
 
 void SparseFactor::factor(cudaStream_t st, int* launches) {
   SparseDev d = d_;
+  if (launches) *launches += 1;
+  if (cta_factor_) {
+    k_sparse_factor_cta<<<1, kCtaThreads, 0, st>>>(d);
+    SOV_LAUNCH_CHECK();
+    return;
+  }
   void* args[] = {&d};
   SOV_CUDA(cudaLaunchCooperativeKernel((const void*)k_sparse_factor, dim3(grid_), dim3(kSparseThreads), args, 0, st));
-  if (launches) *launches += 1;
 }
 
 void SparseFactor::solve(double* z, cudaStream_t st, int* launches, const int* run) {
   SparseDev d = d_;
+  if (launches) *launches += 1;
+  if (cta_solve_) {
+    k_sparse_solve_cta<<<1, kCtaThreads, cta_solve_smem(d.m, d.levels), st>>>(d, z, run);
+    SOV_LAUNCH_CHECK();
+    return;
+  }
   void* args[] = {&d, &z, &run};
   SOV_CUDA(cudaLaunchCooperativeKernel((const void*)k_sparse_solve, dim3(grid_), dim3(kSparseThreads), args, 0, st));
-  if (launches) *launches += 1;
 }
 
 }  // namespace sov

@@ -6,7 +6,8 @@
 // a_ab -= L~_ak L~_bk / D_k. Columns of one level of the elimination tree have no ancestor relation:
 // a level's pivots are taken together, then its rank-1 updates are applied, grouped per destination
 // (each destination's contributions summed by one warp in a fixed order: deterministic). One
-// cooperative launch per factorization and per solve, a grid barrier between levels.
+// launch per factorization and per solve: cooperative over the grid with a grid barrier between
+// levels, or one CTA where the barriers would outweigh the work.
 // Pivot rule of the reference's sparse LDL' (sparse_ldlt.cpp:165-173): a pivot at most
 // drop_tol * |assembled diagonal| (or not finite) marks a dependent row, D = 1e128; with a sign
 // per pivot (quasi-definite systems) the test is sign * pivot, and a dropped pivot keeps its sign.
@@ -22,7 +23,7 @@
 namespace sov {
 
 struct SparseDev {
-  int m, levels;
+  int m, levels, nnz;
   double* V;            // m + nnz(L)
   double* diag;         // m: assembled diagonal (elimination order), the pivot reference
   double* inv_d;        // m
@@ -54,6 +55,7 @@ struct SparseDev {
   const int* up_b;      // updates: position of l_bk
   const int* row_pos;   // entries of L by row (forward solve): positions in L
   const int* row_col;   // their columns
+  double* fval;         // nnz: L~ / D in that order, left by the factorization (null: not wanted)
   int* drop_count;
   int* fail;
   double drop_tol;
@@ -82,6 +84,7 @@ class SparseFactor {
   std::vector<void*> bufs_;
   long long nnz_l_ = 0;
   int grid_ = 1;
+  bool cta_factor_ = false, cta_solve_ = false;  // on one CTA instead of the grid
 };
 
 }  // namespace sov
