@@ -28,6 +28,7 @@
 #include <numeric>
 #include <sstream>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "batch.hpp"
@@ -88,12 +89,13 @@ namespace {
 
 struct CtaScalars {
   double v[16];
-  int flag[4];
+  int flag[4];  // F_*
 };
+enum : int { F_BETTER = 0, F_DONE, F_BEST_IT, F_DROPS };
 
 // scalar slots
 enum : int {
-  S_MU = 0, S_PRES, S_DRES, S_GAP, S_METRIC, S_CX, S_APAFF, S_ADAFF, S_SIGMA, S_AP, S_AD, S_BEST
+  S_MU = 0, S_PRES, S_DRES, S_GAP, S_METRIC, S_CX, S_SIGMA, S_AP, S_AD, S_BEST, S_BGAP, S_BP, S_BD
 };
 
 template <int NT>
@@ -101,12 +103,332 @@ __device__ __forceinline__ void cta_reduce4(double (&v)[4], const int (&ops)[4],
   block_reduce<4>(v, ops, red);
 }
 
+// ---- in-place L D L' (L~ = L D kept unscaled below the diagonal; vinv = 1/D) ----
+// Blocked right-looking over panels of 8 columns. Per panel
+//  (1) one thread per row below the panel's diagonal block runs the column recurrence on its 8
+//      entries held in registers;
+//  (2) warp 0, which has just solved the next 8 rows itself, brings the next diagonal block up to
+//      date and factors it in registers, while the other warps, once all rows are solved, apply the panel's rank-8 update to
+//      the rest of the trailing triangle in 8 x 8 tiles of two FP64 MMAs (m8n8k4) each: an MMA does
+//      256 multiply-adds per issue slot, and a tile takes 6 shared loads and 2 stores per lane where
+//      4 x 4 register tiles took 104 for as much arithmetic.
+// Warp 0 waits for the others once a panel. What bounds the factor is its pivot chain (a shuffle, a
+// reciprocal and two multiply-adds per column) and, with four LPs on an SM, issue slots; the FP64
+// rate itself is far. Measured (m = 100, one LP on the SM): 49 us with warp 0's columns going through
+// shared memory, a barrier after each of three steps and 4 x 4 tiles; 24 us in this form.
+// The order is padded to mp, a multiple of 8, with identity rows (M_ii = 1, vdiag 1), so every block is
+// whole. Row mp holds a right-hand side r: it takes every column's update like any row below the panels,
+// which is the forward substitution, so afterwards M[mp][k] = (L^-1 r)_k and only the backward
+// substitution is left for that right-hand side.
+// Afterwards the strict lower part of every diagonal block holds T = (L_bb)^-1 (unit lower) instead of
+// L~: the solves multiply by it. vdiag holds the assembled diagonal, the reference for the
+// dependent-row test. Returns 1 when a pivot was not finite; *drops_out (shared) counts dependent rows.
+// Not inlined: its registers stay apart from the many pointers of solve_lp; shared memory is named, so
+// that its accesses need no generic addressing.
+__host__ __device__ constexpr int pad8(int m) { return (m + 7) & ~7; }
+
+// the triangle of the block at column k0 into registers (the diagonal too if kDiag)
+template <bool kDiag>
+__device__ __forceinline__ void load_block(const double* M, int k0, double (&d)[8][8]) {
+  const double* row = M + tri(k0) + k0;
+  int step = k0 + 1;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+#pragma unroll
+    for (int c = 0; c < r + (kDiag ? 1 : 0); ++c) d[r][c] = row[c];
+    row += step++;
+  }
+}
+
+template <int NT>
+__device__ __noinline__ int factor_ldl(int mp, int mmax, int* drops_out) {
+  extern __shared__ double sm[];
+  __shared__ int outcome[2];
+  constexpr int NW = NT / 32, KB = 8;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double* const M = sm;
+  double* const vdiag = sm + tri(mmax + 1) + 4 * mmax;
+  double* const vinv = vdiag + mmax;
+  int drops = 0, fail = 0;  // warp 0
+  // The diagonal block at column k0, warp 0: every lane holds the whole triangle and computes the same,
+  // so the chain has no exchanges: a reciprocal and two multiply-adds per column (1270 cycles a block;
+  // 1560 with a row per lane and shuffles). Lane r stores row r.
+  auto factor_diagonal = [&](int k0) {
+    double d[KB][KB], thr[KB], own = 0.0;
+    load_block<true>(M, k0, d);
+#pragma unroll
+    for (int r = 0; r < KB; ++r) thr[r] = 1e-13 * fabs(vdiag[k0 + r]);
+#pragma unroll
+    for (int k = 0; k < KB; ++k) {
+      const double p = d[k][k];
+      double inv = 1.0 / p;
+      // not finite, or a dependent row (sparse_ldlt.cpp:167-173): the pivot is 1e128
+      if (!(p > thr[k] && p <= DBL_MAX)) {
+        inv = 1e-128;
+        if (fabs(p) <= DBL_MAX) ++drops;
+        else fail = 1;
+      }
+      own = lane == k ? inv : own;
+#pragma unroll
+      for (int i = k + 1; i < KB; ++i) {
+        const double lik = d[i][k] * inv;
+#pragma unroll
+        for (int j = k + 1; j <= i; ++j) d[i][j] -= lik * d[j][k];
+      }
+    }
+    if (lane < KB) vinv[k0 + lane] = own;
+    double* row = M + tri(k0 + min(lane, KB - 1)) + k0;
+#pragma unroll
+    for (int c = 0; c < KB; ++c) {
+      double o = d[KB - 1][c];
+#pragma unroll
+      for (int r = KB - 2; r >= c; --r) o = lane == r ? d[r][c] : o;
+      if (lane < KB && c <= lane) row[c] = o;
+    }
+  };
+  // One 8 x 8 tile of a panel's update: lane (q, t) = (lane / 4, lane % 4) holds entries (q, 2t) and
+  // (q, 2t + 1) of it at c, a0, a1 = -L_ik of columns t and 4 + t of the panel, and b0, b1 = L~_jk
+  auto update_tile = [&](double* c, const double* b, double a0, double a1, bool s0, bool s1) {
+    const double b0 = b[0], b1 = b[4];
+    double c0 = c[0], c1 = c[1];
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c0), "+d"(c1) : "d"(a0), "d"(b0));
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c0), "+d"(c1) : "d"(a1), "d"(b1));
+    if (s0) c[0] = c0;
+    if (s1) c[1] = c1;
+  };
+  const int q = lane >> 2, t = lane & 3;
+  if (warp == 0) factor_diagonal(0);
+  __syncthreads();
+  for (int k0 = 0; k0 < mp; k0 += KB) {
+    const int k1 = k0 + KB;
+    // rows k1 .. mp, a thread each
+    if (k1 + tid <= mp) {
+      double f[KB][KB], v[KB];
+      load_block<false>(M, k0, f);
+#pragma unroll
+      for (int a = 0; a < KB; ++a) v[a] = vinv[k0 + a];
+      for (int i = k1 + tid; i <= mp; i += NT) {
+        double r[KB];
+        double* Mi = M + tri(i) + k0;
+#pragma unroll
+        for (int a = 0; a < KB; ++a) r[a] = Mi[a];
+#pragma unroll
+        for (int a = 0; a < KB; ++a) {
+          const double l = r[a] * v[a];
+#pragma unroll
+          for (int c = a + 1; c < KB; ++c) r[c] -= l * f[c][a];
+        }
+#pragma unroll
+        for (int a = 1; a < KB; ++a) Mi[a] = r[a];
+      }
+    }
+    if (k1 == mp) break;  // row mp has taken every column
+    const double v0 = vinv[k0 + t], v1 = vinv[k0 + 4 + t];
+    if (warp == 0) {
+      __syncwarp();
+      asm volatile("bar.arrive 1, %0;" ::"n"(NT) : "memory");  // rows k1 .. k1 + 31 are solved
+      double* row = M + tri(k1 + q);
+      const double a0 = -(row[k0 + t] * v0), a1 = -(row[k0 + 4 + t] * v1);
+      update_tile(row + k1 + 2 * t, row + k0 + t, a0, a1, 2 * t <= q, 2 * t + 1 <= q);
+      __syncwarp();
+      factor_diagonal(k1);
+    } else {
+      asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");  // all rows are solved
+      // strips of 8 rows from the longest, dealt back and forth
+      const int strips = (mp - k1) >> 3;
+      for (int d = 0; d * (NW - 1) < strips - 1; ++d) {
+        const int ib = strips - 1 - d * (NW - 1) - ((d & 1) ? NW - 1 - warp : warp - 1);
+        if (ib <= 0) continue;
+        double* row = M + tri(k1 + 8 * ib + q);
+        const double a0 = -(row[k0 + t] * v0), a1 = -(row[k0 + 4 + t] * v1);
+        double* c = row + k1 + 2 * t;
+        const double* bp = M + tri(k1 + q) + k0 + t;
+        int step = 8 * (k1 + q) + 36;  // tri(j + 8) - tri(j)
+#pragma unroll 2
+        for (int jb = 0; jb < ib; ++jb) {
+          update_tile(c, bp, a0, a1, true, true);
+          c += 8;
+          bp += step;
+          step += 64;
+        }
+        update_tile(c, bp, a0, a1, 2 * t <= q, 2 * t + 1 <= q);
+      }
+      // row mp, a thread per column
+      double* rhs = M + tri(mp);
+      for (int j = k1 + tid - 32; j < mp; j += NT - 32) {
+        const double* Mj = M + tri(j) + k0;
+        double acc = 0.0;
+#pragma unroll
+        for (int a = 0; a < KB; ++a) acc += (rhs[k0 + a] * vinv[k0 + a]) * Mj[a];
+        rhs[j] -= acc;
+      }
+    }
+    __syncthreads();
+  }
+  if (tid == 0) {
+    outcome[0] = fail;
+    outcome[1] = drops;
+  }
+  __syncthreads();
+  // T of every diagonal block, a thread per column: L_bb t = e_c, right-looking
+  if (tid < 128) {  // whole warps: blocks of one warp may lie past mp
+    const int k0 = (tid >> 3) * KB, c = tid & 7;
+    double x[KB];
+    if (k0 < mp) {
+      double f[KB][KB], v[KB];
+      load_block<false>(M, k0, f);
+#pragma unroll
+      for (int r = 0; r < KB; ++r) {
+        v[r] = vinv[k0 + r];
+        x[r] = r == c ? 1.0 : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < KB - 1; ++k) {
+        const double w = x[k] * v[k];
+#pragma unroll
+        for (int r = k + 1; r < KB; ++r) x[r] -= f[r][k] * w;
+      }
+    }
+    __syncwarp();
+    if (k0 < mp) {
+#pragma unroll
+      for (int r = 1; r < KB; ++r)
+        if (r > c) M[tri(k0 + r) + k0 + c] = x[r];
+    }
+  }
+  if (tid == 0) *drops_out += outcome[1];
+  const int failed = outcome[0];
+  __syncthreads();
+  return failed;
+}
+
+// ---- solve L D L' z = rhs in place (warp 0) ----
+// Lane l holds rows l, l + 32, l + 64, l + 96 of z (and of 1/D) in registers. Blocks of eight columns:
+// the block's eight values are exchanged by shuffles, multiplied by T = (L_bb)^-1 (forward) or its
+// transpose (backward), and after a second exchange the other rows take the eight terms: forward
+// z_i -= L~_ik w_k (w = y / D), backward a_i += L~_ki x_k with x = w - a / D. Per block the chain is two
+// exchanges and some ten multiply-adds, where a column at a time took a shuffle and two dependent
+// multiply-adds for each of the eight columns (m = 100: both directions 11.8 -> 10.3 us).
+// fwd_done: the forward substitution was done by the factorization (row mp of M holds L^-1 rhs), so
+// w = D^-1 (row mp) and only the backward substitution runs. Rows m .. mp - 1 are the padding.
+template <bool fwd_done>
+__device__ __noinline__ void solve_ldl(int m, int mmax) {
+  extern __shared__ double sm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, mp = pad8(m);
+  double* const M = sm;
+  double* const vz = sm + tri(mmax + 1) + 2 * mmax;
+  double* const vinv = sm + tri(mmax + 1) + 5 * mmax;
+  if (warp == 0) {
+    double zr[4], ir[4], ar[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = u * 32 + lane;
+      ir[u] = i < mp ? vinv[i] : 0.0;
+      zr[u] = i < m ? (fwd_done ? M[tri(mp) + i] * ir[u] : vz[i]) : 0.0;
+      ar[u] = 0.0;
+    }
+    if (!fwd_done) {
+      const double* row[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) row[u] = M + tri(min(u * 32 + lane, mp));
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        if (g * 32 >= mp) break;
+        const int kend = min(32, mp - g * 32);
+        for (int kb = 0; kb < kend; kb += 8) {
+          const int k0 = g * 32 + kb;
+          // the lane's entries of the block's columns (rows of the group above the block: none)
+          double l[4][8], s[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const double v = row[g][lane > kb + e ? k0 + e : 0];
+            l[g][e] = lane > kb + e ? v : 0.0;
+          }
+#pragma unroll
+          for (int u = g + 1; u < 4; ++u)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) l[u][e] = row[u][k0 + e];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) s[e] = __shfl_sync(kFull, zr[g], kb + e);
+          double y0 = zr[g], y1 = 0.0;
+#pragma unroll
+          for (int e = 0; e < 8; e += 2) {
+            y0 += l[g][e] * s[e];
+            y1 += l[g][e + 1] * s[e + 1];
+          }
+          const double w = (y0 + y1) * ir[g];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) s[e] = __shfl_sync(kFull, w, kb + e);
+#pragma unroll
+          for (int u = g; u < 4; ++u) {
+            double a0 = 0.0, a1 = 0.0;
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+              a0 += l[u][e] * s[e];
+              a1 += l[u][e + 1] * s[e + 1];
+            }
+            const double rest = zr[u] - (a0 + a1);
+            zr[u] = u == g && lane >= kb && lane < kb + 8 ? w : rest;
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int g = 3; g >= 0; --g) {
+      if (g * 32 >= mp) continue;
+      for (int kb = min(32, mp - g * 32) - 8; kb >= 0; kb -= 8) {
+        const int k0 = g * 32 + kb;
+        double l[4][8], s[8];
+        const double* row = M + tri(k0);
+        int step = k0 + 1;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+#pragma unroll
+          for (int u = 0; u < g; ++u) l[u][e] = row[u * 32 + lane];
+          const double v = row[lane < kb + e ? g * 32 + lane : 0];
+          l[g][e] = lane < kb + e ? v : 0.0;
+          row += step++;
+        }
+        const double v = zr[g] - ir[g] * ar[g];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] = __shfl_sync(kFull, v, kb + e);
+        double x0 = v, x1 = 0.0;
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+          x0 += l[g][e] * s[e];
+          x1 += l[g][e + 1] * s[e + 1];
+        }
+        const double x = x0 + x1;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] = __shfl_sync(kFull, x, kb + e);
+        zr[g] = lane >= kb && lane < kb + 8 ? x : zr[g];
+#pragma unroll
+        for (int u = 0; u <= g; ++u) {
+          double a0 = ar[u], a1 = 0.0;
+#pragma unroll
+          for (int e = 0; e < 8; e += 2) {
+            a0 += l[u][e] * s[e];
+            a1 += l[u][e + 1] * s[e + 1];
+          }
+          ar[u] = a0 + a1;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = u * 32 + lane;
+      if (i < m) vz[i] = zr[u];
+    }
+  }
+  __syncthreads();
+}
+
 template <int NT>
 __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* sm, int mmax, double* red,
                          CtaScalars& cs) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NW = NT / 32;
-  const int m = mt.m, n = mt.n;
+  const int m = mt.m, n = mt.n, mp = pad8(m);
   // M: lower triangle, packed by rows (row i at tri(i)); then six m-vectors
   double* M = sm;
   double* vy = sm + tri(mmax + 1);
@@ -117,27 +439,35 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
   double* vinv = vdiag + mmax;
   int* srp = reinterpret_cast<int*>(vinv + mmax);  // the row pointers (m + 1), read by every row pass
 
-  const int* ri = bd.row_idx + mt.a_off;
-  const double* cv = bd.cval + mt.a_off;
-  const int* rpp = bd.row_ptr + mt.rp_off;
-  const int* ci = bd.col_idx + mt.a_off;
-  const double* rv = bd.rval + mt.a_off;
-  const int4* crc = bd.crec + mt.nv_off;
-  const double2* cv2 = bd.cval2 + mt.nv_off;
-  const double* b = bd.b + mt.mv_off;
-  const double* c = bd.c + mt.nv_off;
-  double* x = bd.x + mt.nv_off;
-  double* s = bd.s + mt.nv_off;
-  double* dx = bd.dx + mt.nv_off;
-  double* ds = bd.ds + mt.nv_off;
-  double* dxa = bd.dxa + mt.nv_off;
-  double* dsa = bd.dsa + mt.nv_off;
-  double* rd = bd.rd + mt.nv_off;
-  double* bx = bd.bx + mt.nv_off;
-  double* bs = bd.bs + mt.nv_off;
-  double* gy = bd.y + mt.mv_off;
-  double* gby = bd.by + mt.mv_off;
-  int drops = 0, fail = 0;
+  // The LP's arrays are formed from these offsets where a pass uses them, and the offsets are made
+  // opaque at every call of the factor and the solves (forget_pointers): pointers held across them
+  // (20 of them) are spilled, and with four LPs' triangles in shared memory an SM has little L1 left
+  // for spills (4096 transportation LPs at 128 threads: 17.4 ms with them, 17.0 ms without; at 256 threads 14.7 and 13.3 ms).
+  long long a_off = mt.a_off, nv_off = mt.nv_off, mv_off = mt.mv_off;
+  auto forget_pointers = [&]() { asm volatile("" : "+l"(a_off), "+l"(nv_off), "+l"(mv_off)); };
+#define LP_ARRAY(type, name, expr) auto name = [&]() -> type { return expr; }
+  LP_ARRAY(const int*, ri, bd.row_idx + a_off);
+  LP_ARRAY(const double*, cv, bd.cval + a_off);
+  LP_ARRAY(const int*, ci, bd.col_idx + a_off);
+  LP_ARRAY(const double*, rv, bd.rval + a_off);
+  LP_ARRAY(const int4*, crc, bd.crec + nv_off);
+  LP_ARRAY(const double2*, cv2, bd.cval2 + nv_off);
+  LP_ARRAY(const double*, b, bd.b + mv_off);
+  LP_ARRAY(const double*, c, bd.c + nv_off);
+  LP_ARRAY(double*, x, bd.x + nv_off);
+  LP_ARRAY(double*, s, bd.s + nv_off);
+  LP_ARRAY(double*, dx, bd.dx + nv_off);
+  LP_ARRAY(double*, ds, bd.ds + nv_off);
+  LP_ARRAY(double*, dxa, bd.dxa + nv_off);
+  LP_ARRAY(double*, dsa, bd.dsa + nv_off);
+  LP_ARRAY(double*, rd, bd.rd + nv_off);
+  LP_ARRAY(double*, bx, bd.bx + nv_off);
+  LP_ARRAY(double*, bs, bd.bs + nv_off);
+  LP_ARRAY(double*, gy, bd.y + mv_off);
+  LP_ARRAY(double*, gby, bd.by + mv_off);
+#undef LP_ARRAY
+  int fail = 0;
+  if (tid == 0) cs.flag[F_DROPS] = 0;
 
   // ---- normal matrix M = A diag(d) A' + 1e-12 I, assembled inside the residual passes ----
   // Off-diagonal entries come from the column pass: thread per column j, one shared-memory atomic
@@ -147,11 +477,11 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
   // M is cleared by the pass before (start-up, or the update of the previous iteration).
   auto offdiag = [&](int pb, int pe, double dj) {
     for (int qa = pb; qa < pe; ++qa) {
-      const int ra = ri[qa];
-      const double va = cv[qa] * dj;
+      const int ra = ri()[qa];
+      const double va = cv()[qa] * dj;
       for (int qb = pb; qb < pe; ++qb) {
-        const int rb = ri[qb];
-        if (rb < ra) atomicAdd(M + tri(ra) + rb, va * cv[qb]);
+        const int rb = ri()[qb];
+        if (rb < ra) atomicAdd(M + tri(ra) + rb, va * cv()[qb]);
       }
     }
   };
@@ -174,8 +504,10 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
   //  mode 2 (corrector): z = rp + A t with t = tv - smu dv (tv = t0, dv = w of the predictor pass)
   // Returns this thread's share of max |rp_i| (mode 1).
   constexpr int RW = 3;
-  auto row_pass = [&](const int mode, const double* dv, const double* tv, double smu = 0.0) {
+  auto row_pass = [&](auto mode_c, const double* dv, const double* tv, double smu = 0.0) {
+    constexpr int mode = decltype(mode_c)::value;
     double rpm = 0.0;
+    if (mode != 2 && tid < mp - m) M[tri(m + tid) + m + tid] = 1.0;  // the padding rows
     for (int i0 = warp; i0 < m; i0 += RW * NW) {
       int rows[RW], pb[RW], pe[RW];
       double g0[RW], g1[RW], g2[RW];
@@ -188,28 +520,52 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
         len = max(len, pe[h] - pb[h]);
         g0[h] = g1[h] = g2[h] = 0.0;
       }
-      for (int o = lane; o < len; o += 32) {
+      // chunks of 32 entries of each row, two at a time where a row has more than one, their loads issued
+      // before any is used: the entries (value, column), then what they gather; a lane past its row's
+      // end adds zeros
+      auto chunks = [&](auto uc) {
+        constexpr int U2 = decltype(uc)::value;
+      for (int o = lane; o < len; o += 32 * U2) {
+        double a[RW][U2], gx[RW][U2], gd[RW][U2], gt[RW][U2];
+        int k[RW][U2];
 #pragma unroll
-        for (int h = 0; h < RW; ++h) {
-          const int p = pb[h] + o;
-          if (p < pe[h]) {
-            const double a = rv[p];
+        for (int h = 0; h < RW; ++h)
+#pragma unroll
+          for (int u = 0; u < U2; ++u) {
+            const int p = pb[h] + o + 32 * u;
+            const bool on = p < pe[h];
+            a[h][u] = on ? rv()[p] : 0.0;
+            k[h][u] = on && mode != 0 ? ci()[p] : -1;
+          }
+#pragma unroll
+        for (int h = 0; h < RW; ++h)
+#pragma unroll
+          for (int u = 0; u < U2; ++u) {
+            const int kk = k[h][u];
+            gx[h][u] = mode == 1 && kk >= 0 ? x()[kk] : 0.0;
+            gd[h][u] = mode != 0 && kk >= 0 ? dv[kk] : 0.0;
+            gt[h][u] = mode != 0 && kk >= 0 ? tv[kk] : 0.0;
+          }
+#pragma unroll
+        for (int u = 0; u < U2; ++u)
+#pragma unroll
+          for (int h = 0; h < RW; ++h) {
+            const double v = a[h][u];
             if (mode == 0) {
-              g0[h] += a;
-              g1[h] += a * a;
+              g0[h] += v;
+              g1[h] += v * v;
+            } else if (mode == 1) {
+              g0[h] += v * gx[h][u];
+              g1[h] += v * v * gd[h][u];
+              g2[h] += v * gt[h][u];
             } else {
-              const int k = ci[p];
-              if (mode == 1) {
-                g0[h] += a * x[k];
-                g1[h] += a * a * dv[k];
-                g2[h] += a * tv[k];
-              } else {
-                g2[h] += a * (tv[k] - smu * dv[k]);
-              }
+              g2[h] += v * (gt[h][u] - smu * gd[h][u]);
             }
           }
-        }
       }
+      };
+      if (len > 32) chunks(std::integral_constant<int, 2>{});
+      else chunks(std::integral_constant<int, 1>{});
 #pragma unroll
       for (int h = 0; h < RW; ++h) {
         const double s0 = mode != 2 ? warp_sum(g0[h]) : 0.0;
@@ -221,7 +577,7 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
           if (lane == 0) vz[i] = vrp[i] + s2;
           continue;
         }
-        const double r = b[i] - s0;
+        const double r = b()[i] - s0;
         if (mode == 1) rpm = fmax(rpm, fabs(r));
         if (lane == 0) {
           M[tri(i) + i] = s1 + 1e-12;
@@ -229,185 +585,18 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
           const double rhs = mode == 1 ? r + s2 : r;
           if (mode == 1) vrp[i] = r;
           vz[i] = rhs;
-          M[tri(m) + i] = rhs;  // the augmented row of the factorization that follows
+          M[tri(mp) + i] = rhs;  // the augmented row of the factorization that follows
         }
       }
     }
     return rpm;
   };
 
-  // ---- in-place L D L' (L~ = L D kept unscaled below the diagonal; vinv = 1/D) ----
-  // Blocked right-looking over panels of KB columns, three barriers per panel:
-  //  (1) warp 0 factors the KB x KB diagonal block, lane = row, one column at a time;
-  //  (2) one thread per row below the block runs the same column recurrence on its KB panel
-  //      entries held in registers;
-  //  (3) the trailing lower triangle takes the panel's rank-KB update in 4 x 4 register tiles
-  //      (8 shared loads per 16 FMAs instead of 3 shared accesses per FMA).
-  // Every entry sees the same operations in the same order as the column-at-a-time algorithm
-  // (M[i][j] -= (M[i][k] / D_k) * M[j][k] for k = 0, 1, ...), so the factor is bit-identical to it.
-  // With `augmented`, row m holds a right-hand side r: it takes every column's update like any row
-  // below the panels, which is the forward substitution, so afterwards M[m][k] = (L^-1 r)_k and
-  // only the backward substitution is left for that right-hand side.
-  // vdiag[k] (the assembled diagonal, the reference for the dependent-row test) is overwritten
-  // with the pivot outcome of column k once it has been used: 0 kept, 1 dropped, 2 not finite.
-  auto factor = [&](bool augmented) {
-    constexpr int KB = 8;
-    const int mr = augmented ? m + 1 : m;  // rows factored: row m carries a right-hand side
-    for (int k0 = 0; k0 < m; k0 += KB) {
-      const int k1 = min(k0 + KB, m);
-      if (warp == 0) {
-        for (int k = k0; k < k1; ++k) {
-          const double p = M[tri(k) + k];
-          const double dref = vdiag[k];
-          // 2: not finite, 1: dependent row (sparse_ldlt.cpp:167-173), 0: kept; no branches
-          const double code = !(fabs(p) <= DBL_MAX) ? 2.0 : (p <= 1e-13 * fabs(dref) ? 1.0 : 0.0);
-          const double inv = 1.0 / (code != 0.0 ? 1e128 : p);
-          const int i = k + 1 + lane;
-          if (i < k1) {
-            const double lik = M[tri(i) + k] * inv;
-            double* Mi = M + tri(i);
-            for (int j = k + 1; j <= i; ++j) Mi[j] -= lik * M[tri(j) + k];
-          }
-          __syncwarp();
-          if (lane == 0) {
-            vinv[k] = inv;
-            vdiag[k] = code;
-          }
-        }
-      }
-      __syncthreads();
-      for (int k = k0; k < k1; ++k) {
-        const double code = vdiag[k];
-        if (code == 1.0) ++drops;
-        if (code == 2.0) fail = 1;
-      }
-      for (int i = k1 + tid; i < mr; i += NT) {
-        double r[KB];
-        double* Mi = M + tri(i) + k0;
-#pragma unroll
-        for (int a = 0; a < KB; ++a) r[a] = k0 + a < k1 ? Mi[a] : 0.0;
-#pragma unroll
-        for (int a = 0; a < KB; ++a) {
-          if (k0 + a < k1) {
-            const double l = r[a] * vinv[k0 + a];
-#pragma unroll
-            for (int c = a + 1; c < KB; ++c)
-              if (k0 + c < k1) r[c] -= l * M[tri(k0 + c) + k0 + a];
-          }
-        }
-#pragma unroll
-        for (int a = 0; a < KB; ++a)
-          if (k0 + a < k1) Mi[a] = r[a];
-      }
-      __syncthreads();
-      const int tt = (mr - k1 + 3) >> 2;
-      const int ntiles = tt * (tt + 1) / 2;
-      for (int tile = tid; tile < ntiles; tile += NT) {
-        int ti = static_cast<int>((sqrtf(8.0f * tile + 1.0f) - 1.0f) * 0.5f);
-        while (ti * (ti + 1) / 2 > tile) --ti;
-        while ((ti + 1) * (ti + 2) / 2 <= tile) ++ti;
-        const int tj = tile - ti * (ti + 1) / 2;
-        const int i0 = k1 + 4 * ti, j0 = k1 + 4 * tj;
-        // rows past mr are clamped to mr - 1 and columns to the row (in-bounds loads, stores masked)
-        int ri4[4], rj4[4], iq[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          iq[q] = min(i0 + q, mr - 1);
-          ri4[q] = tri(iq[q]);
-          rj4[q] = tri(min(j0 + q, mr - 1));
-        }
-        double acc[4][4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-          for (int r = 0; r < 4; ++r) acc[q][r] = M[ri4[q] + min(j0 + r, iq[q])];
-        for (int k = k0; k < k1; ++k) {
-          const double inv = vinv[k];
-          double li[4], lj[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            li[q] = M[ri4[q] + k] * inv;
-            lj[q] = M[rj4[q] + k];
-          }
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int r = 0; r < 4; ++r) acc[q][r] -= li[q] * lj[r];
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-          for (int r = 0; r < 4; ++r)
-            if (i0 + q < mr && j0 + r <= i0 + q) M[ri4[q] + j0 + r] = acc[q][r];
-      }
-      __syncthreads();
-    }
-  };
-
-  // ---- solve L D L' z = rhs in place (warp 0) ----
-  // Lane l holds rows l, l + 32, l + 64, l + 96 of z (and of 1/D) in registers; step k broadcasts
-  // the finished entry with a shuffle, so the serial chain per step is shuffle + FMA with the
-  // shared-memory loads of L~ off the chain. Same operations, in the same order, as the
-  // row-at-a-time substitution: forward w_k = z_k / D_k, z_i -= L~_ik w_k (L~ = L D); backward
-  // x_k = w_k - (1/D_k) sum_{j>k} L~_jk x_j.
-  // fwd_done: the forward substitution was done by an augmented factorization (row m of M holds
-  // L^-1 rhs), so w = D^-1 (row m) and only the backward substitution runs.
-  auto solve = [&](bool fwd_done) {
-    if (warp == 0) {
-      double zr[4], ir[4], ar[4];
-      int ro[4];
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int i = t * 32 + lane;
-        ir[t] = i < m ? vinv[i] : 0.0;
-        zr[t] = i < m ? (fwd_done ? M[tri(m) + i] * ir[t] : vz[i]) : 0.0;
-        ar[t] = 0.0;
-        ro[t] = tri(min(i, m - 1));
-      }
-#pragma unroll
-      for (int t = 0; t < 4 && !fwd_done; ++t) {
-        const int kend = min(32, m - t * 32);
-        for (int kk = 0; kk < kend; ++kk) {
-          const int k = t * 32 + kk;
-          const double wk = __shfl_sync(0xffffffffu, zr[t], kk) * __shfl_sync(0xffffffffu, ir[t], kk);
-          if (lane == kk) zr[t] = wk;
-#pragma unroll
-          for (int u = t; u < 4; ++u) {
-            const int i = u * 32 + lane;
-            if (i > k && i < m) zr[u] -= M[ro[u] + k] * wk;
-          }
-        }
-      }
-#pragma unroll
-      for (int t = 3; t >= 0; --t) {
-        const int kstart = min(31, m - 1 - t * 32);
-        for (int kk = kstart; kk >= 0; --kk) {
-          const int k = t * 32 + kk;
-          const double own = zr[t] - ir[t] * ar[t];
-          const double xk = __shfl_sync(0xffffffffu, own, kk);
-          if (lane == kk) zr[t] = xk;
-          const int rk = tri(k);
-#pragma unroll
-          for (int u = 0; u <= t; ++u) {
-            const int i = u * 32 + lane;
-            if (i < k) ar[u] += M[rk + i] * xk;
-          }
-        }
-      }
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int i = t * 32 + lane;
-        if (i < m) vz[i] = zr[t];
-      }
-    }
-    __syncthreads();
-  };
-
   // sum_p a_pj v[row_p] over column j from its record: the first two entries (missing ones as
   // 0 * v[0]) need no load that waits on another, the rest of a longer column follows from col_ptr
   auto col_dot = [&](const int4 rc, const double2 av, const double* v) {
     double acc = av.x * v[rc.x] + av.y * v[rc.y];
-    for (int p = rc.z + 2; p < rc.w; ++p) acc += cv[p] * v[ri[p]];
+    for (int p = rc.z + 2; p < rc.w; ++p) acc += cv()[p] * v[ri()[p]];
     return acc;
   };
   constexpr int U = 3;  // columns per thread per pass, loads issued before use
@@ -416,41 +605,44 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
   // per-column scratch of an iteration: d = x/s in ds and t = d rd - rxs/s in dx for the
   // predictor's row pass, then w = 1/s in ds and t0 in dx for the corrector's (both free between
   // the update of one iteration and the corrector's direction pass that overwrites them)
-  double* dvec = ds;
-  double* tvec = dx;
+  auto dvec = [&]() { return ds(); };
+  auto tvec = [&]() { return dx(); };
   auto mehrotra_start = [&]() {
-    for (int i = tid; i < tri(m + 1); i += NT) M[i] = 0.0;
+    for (int i = tid; i < tri(mp + 1); i += NT) M[i] = 0.0;
     __syncthreads();
-    for (int j = tid; j < n; j += NT) offdiag_rec(crc[j], cv2[j], 1.0);
+    for (int j = tid; j < n; j += NT) offdiag_rec(crc()[j], cv2()[j], 1.0);
     __syncthreads();
-    row_pass(0, nullptr, nullptr);
+    row_pass(std::integral_constant<int, 0>{}, nullptr, nullptr);
     __syncthreads();
-    factor(true);
-    solve(true);
+    forget_pointers();
+    fail |= factor_ldl<NT>(mp, mmax, &cs.flag[F_DROPS]);
+    solve_ldl<true>(m, mmax);
+    forget_pointers();
     const bool start_ok = !fail;
     for (int j = tid; j < n; j += NT) {
       double xs = 1.0, ss = 1.0;
       if (start_ok) {
         double atdy = 0.0;
-        const int4 rc = crc[j];
-        for (int p = rc.z; p < rc.w; ++p) atdy += cv[p] * vz[ri[p]];
+        const int4 rc = crc()[j];
+        for (int p = rc.z; p < rc.w; ++p) atdy += cv()[p] * vz[ri()[p]];
         xs = fmax(1.0, fabs(atdy));
-        ss = fmax(1.0, fabs(c[j] - atdy));
+        ss = fmax(1.0, fabs(c()[j] - atdy));
       }
-      x[j] = xs;
-      s[j] = ss;
-      bx[j] = xs;
-      bs[j] = ss;
+      x()[j] = xs;
+      s()[j] = ss;
+      bx()[j] = xs;
+      bs()[j] = ss;
     }
     for (int i = tid; i < m; i += NT) {
       vy[i] = start_ok ? vz[i] : 0.0;
-      gby[i] = vy[i];
+      gby()[i] = vy[i];
     }
-    for (int i = tid; i < tri(m + 1); i += NT) M[i] = 0.0;
+    for (int i = tid; i < tri(mp + 1); i += NT) M[i] = 0.0;
     fail = 0;
     __syncthreads();
   };
-  for (int i = tid; i <= m; i += NT) srp[i] = rpp[i];  // visible after mehrotra_start's first barrier
+  for (int i = tid; i <= m; i += NT) srp[i] = bd.row_ptr[mt.rp_off + i];
+  if (tid < mp - m) vdiag[m + tid] = 1.0;  // visible after mehrotra_start's first barrier
   mehrotra_start();
 
   const int ops_res[4] = {1, 1, 0, 0};
@@ -464,16 +656,16 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
       double rpm = 0.0;
       for (int i = warp; i < m; i += NW) {
         double acc = 0.0;
-        for (int p = srp[i] + lane; p < srp[i + 1]; p += 32) acc += rv[p] * x[ci[p]];
+        for (int p = srp[i] + lane; p < srp[i + 1]; p += 32) acc += rv()[p] * x()[ci()[p]];
         acc = warp_sum(acc);
-        rpm = fmax(rpm, fabs(b[i] - acc));
+        rpm = fmax(rpm, fabs(b()[i] - acc));
       }
       double rdm = 0.0, xs = 0.0, cx = 0.0;
       for (int j = tid; j < n; j += NT) {
-        const double r = c[j] - (col_dot(crc[j], cv2[j], vy) + s[j]);
+        const double r = c()[j] - (col_dot(crc()[j], cv2()[j], vy) + s()[j]);
         rdm = fmax(rdm, fabs(r));
-        xs += x[j] * s[j];
-        cx += c[j] * x[j];
+        xs += x()[j] * s()[j];
+        cx += c()[j] * x()[j];
       }
       double v[4] = {rpm, rdm, xs, cx};
       cta_reduce4<NT>(v, ops_res, red);
@@ -490,8 +682,8 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
     point_metric(met_d, mu_d);
     const double* wx = bd.warm + mt.w_off;
     for (int j = tid; j < n; j += NT) {
-      x[j] = wx[j];
-      s[j] = wx[n + m + j];
+      x()[j] = wx[j];
+      s()[j] = wx[n + m + j];
     }
     for (int i = tid; i < m; i += NT) vy[i] = wx[n + i];
     __syncthreads();
@@ -500,18 +692,23 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
       warm_used = 1;
     } else {
       for (int j = tid; j < n; j += NT) {
-        x[j] = bx[j];
-        s[j] = bs[j];
+        x()[j] = bx()[j];
+        s()[j] = bs()[j];
       }
-      for (int i = tid; i < m; i += NT) vy[i] = gby[i];
+      for (int i = tid; i < m; i += NT) vy[i] = gby()[i];
     }
     __syncthreads();
   }
 
-  double best_metric = INFINITY, best_gap = INFINITY, best_p = INFINITY, best_d = INFINITY;
-  int best_it = 0;
+  // the scalars of the loop live in shared memory, kept by thread 0
+  auto reset_best = [&]() {
+    if (tid == 0) {
+      cs.v[S_BEST] = cs.v[S_BGAP] = cs.v[S_BP] = cs.v[S_BD] = INFINITY;
+      cs.flag[F_BEST_IT] = 0;
+    }
+  };
+  reset_best();
   int status = -1, iters = 0;
-  double last_gap = 0, last_p = 0, last_d = 0, last_cx = 0;
   for (int it = 0; it < mt.max_iter; ++it) {
     // residuals, with the predictor's right-hand side and the normal matrix built in the same two
     // passes (interior_point.cpp:572-582, :418-432, :74-101)
@@ -523,11 +720,11 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int j = min(j0 + u * NT, n - 1);
-        rc[u] = crc[j];
-        av[u] = cv2[j];
-        xv[u] = x[j];
-        sv[u] = s[j];
-        cvv[u] = c[j];
+        rc[u] = crc()[j];
+        av[u] = cv2()[j];
+        xv[u] = x()[j];
+        sv[u] = s()[j];
+        cvv[u] = c()[j];
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) aty[u] = col_dot(rc[u], av[u], vy);
@@ -536,20 +733,20 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
         const int j = j0 + u * NT;
         if (j >= n) continue;
         const double r = cvv[u] - (aty[u] + sv[u]);
-        rd[j] = r;
+        rd()[j] = r;
         rdm = fmax(rdm, fabs(r));
         xs += xv[u] * sv[u];
         cx += cvv[u] * xv[u];
         const double xj = fmax(xv[u], 1e-16), sj = fmax(sv[u], 1e-16);
         const double dj = xj / sj;
         const double rxs = -xv[u] * sv[u];
-        dvec[j] = dj;
-        tvec[j] = dj * r - rxs / sj;
+        dvec()[j] = dj;
+        tvec()[j] = dj * r - rxs / sj;
         offdiag_rec(rc[u], av[u], dj);
       }
     }
     __syncthreads();
-    const double rpm = row_pass(1, dvec, tvec);
+    const double rpm = row_pass(std::integral_constant<int, 1>{}, dvec(), tvec());
     double v[4] = {rpm, rdm, xs, cx};
     cta_reduce4<NT>(v, ops_res, red);
     if (tid == 0) {
@@ -560,30 +757,29 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
       cs.v[S_PRES] = pres;
       cs.v[S_DRES] = dres;
       cs.v[S_GAP] = gap;
-      cs.v[S_METRIC] = fmax(pres, fmax(dres, gap));
       cs.v[S_CX] = v[3];
+      const double metric = fmax(pres, fmax(dres, gap));
+      const bool better = metric < cs.v[S_BEST];
+      if (better) {
+        cs.v[S_BEST] = metric;
+        cs.v[S_BGAP] = gap;
+        cs.v[S_BP] = pres;
+        cs.v[S_BD] = dres;
+        cs.flag[F_BEST_IT] = it + 1;
+      }
+      if (gap < cs.v[S_BGAP]) cs.v[S_BGAP] = gap;
+      cs.flag[F_BETTER] = better;
+      cs.flag[F_DONE] = pres < mt.ftol && dres < mt.ftol && gap < mt.otol;
     }
     __syncthreads();
-    const double mu = cs.v[S_MU], pres = cs.v[S_PRES], dres = cs.v[S_DRES], gap = cs.v[S_GAP];
-    const double metric = cs.v[S_METRIC];
-    last_gap = gap;
-    last_p = pres;
-    last_d = dres;
-    last_cx = cs.v[S_CX];
-    if (metric < best_metric) {
-      best_metric = metric;
-      best_gap = gap;
-      best_p = pres;
-      best_d = dres;
-      best_it = it + 1;
+    if (cs.flag[F_BETTER]) {
       for (int j = tid; j < n; j += NT) {
-        bx[j] = x[j];
-        bs[j] = s[j];
+        bx()[j] = x()[j];
+        bs()[j] = s()[j];
       }
-      for (int i = tid; i < m; i += NT) gby[i] = vy[i];
+      for (int i = tid; i < m; i += NT) gby()[i] = vy[i];
     }
-    if (gap < best_gap) best_gap = gap;
-    if (pres < mt.ftol && dres < mt.ftol && gap < mt.otol) {
+    if (cs.flag[F_DONE]) {
       status = SOV_OPTIMAL;
       iters = it + 1;
       break;
@@ -594,13 +790,13 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
     if (warm_used == 1 && it + 1 == kWarmGiveUp) {
       mehrotra_start();
       warm_used = 2;
-      best_metric = best_gap = best_p = best_d = INFINITY;
-      best_it = 0;
+      reset_best();
       continue;
     }
     // factor A diag(x/s) A' (assembled by the residual passes), with the predictor's right-hand
     // side as the augmented row
-    factor(true);
+    forget_pointers();
+    fail |= factor_ldl<NT>(mp, mmax, &cs.flag[F_DROPS]);
     if (fail) {
       status = -2;  // factorization failure: best iterate
       break;
@@ -614,14 +810,17 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
     //    is t0 - sigma mu w, formed inside the row pass z = rp + A t;
     //  corrector: that row pass, solve, one column pass for the direction and the step lengths.
     for (int pass = 0; pass < 2; ++pass) {
-      const double sigma_mu = pass ? cs.v[S_SIGMA] * mu : 0.0;
+      const double sigma_mu = pass ? cs.v[S_SIGMA] * cs.v[S_MU] : 0.0;
       if (pass == 1) {
-        row_pass(2, dvec, tvec, sigma_mu);
+        row_pass(std::integral_constant<int, 2>{}, dvec(), tvec(), sigma_mu);
         __syncthreads();
       }
-      solve(pass == 0);
-      double* ddx = pass ? dx : dxa;
-      double* dds = pass ? ds : dsa;
+      forget_pointers();
+      if (pass == 0) solve_ldl<true>(m, mmax);
+      else solve_ldl<false>(m, mmax);
+      forget_pointers();
+      double* ddx = pass ? dx() : dxa();
+      double* dds = pass ? ds() : dsa();
       double rpmin = 1.0, rdmin = 1.0, sxs = 0.0, sdxs = 0.0, sxds = 0.0, sdd = 0.0;
       for (int j0 = tid; j0 < n; j0 += U * NT) {
         int4 rc[U];
@@ -630,13 +829,13 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           const int j = min(j0 + u * NT, n - 1);
-          rc[u] = crc[j];
-          cav[u] = cv2[j];
-          xv[u] = x[j];
-          sv[u] = s[j];
-          rdv[u] = rd[j];
-          av[u] = pass ? dxa[j] : 0.0;
-          bv[u] = pass ? dsa[j] : 0.0;
+          rc[u] = crc()[j];
+          cav[u] = cv2()[j];
+          xv[u] = x()[j];
+          sv[u] = s()[j];
+          rdv[u] = rd()[j];
+          av[u] = pass ? dxa()[j] : 0.0;
+          bv[u] = pass ? dsa()[j] : 0.0;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) atdy[u] = col_dot(rc[u], cav[u], vz);
@@ -659,8 +858,8 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
             sdxs += dxj * sj;
             sxds += xj * dsj;
             sdd += dxj * dsj;
-            tvec[j] = dj * rdv[u] + (xj * sj + dxj * dsj) / sg;
-            dvec[j] = 1.0 / sg;
+            tvec()[j] = dj * rdv[u] + (xj * sj + dxj * dsj) / sg;
+            dvec()[j] = 1.0 / sg;
           }
         }
       }
@@ -670,10 +869,8 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
         block_reduce<6>(u, ops, red);
         if (tid == 0) {
           const double apa = u[0], ada = u[1];
-          cs.v[S_APAFF] = apa;
-          cs.v[S_ADAFF] = ada;
           const double mu_aff = fmax(0.0, u[2] + apa * u[3] + ada * u[4] + apa * ada * u[5]) / n;
-          const double r = mu_aff / mu;
+          const double mu = cs.v[S_MU], r = mu_aff / mu;
           cs.v[S_SIGMA] = mu > 0.0 ? fmin(1.0, r * r * r) : 0.0;
         }
       } else {
@@ -694,47 +891,47 @@ __device__ void solve_lp(const BatchDev& bd, const LpMeta& mt, int lp, double* s
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int j = min(j0 + u * NT, n - 1);
-        xv[u] = x[j];
-        sv[u] = s[j];
-        av[u] = dx[j];
-        bv[u] = ds[j];
+        xv[u] = x()[j];
+        sv[u] = s()[j];
+        av[u] = dx()[j];
+        bv[u] = ds()[j];
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int j = j0 + u * NT;
         if (j >= n) continue;
-        x[j] = fmax(xv[u] + ap * av[u], 1e-14);
-        s[j] = fmax(sv[u] + ad * bv[u], 1e-14);
+        x()[j] = fmax(xv[u] + ap * av[u], 1e-14);
+        s()[j] = fmax(sv[u] + ad * bv[u], 1e-14);
       }
     }
     for (int i = tid; i < m; i += NT) vy[i] += ad * vz[i];
-    for (int i = tid; i < tri(m + 1); i += NT) M[i] = 0.0;
+    for (int i = tid; i < tri(mp + 1); i += NT) M[i] = 0.0;
     iters = it + 1;
     __syncthreads();
   }
-  for (int i = tid; i < m; i += NT) gy[i] = vy[i];
+  for (int i = tid; i < m; i += NT) gy()[i] = vy[i];
   if (tid == 0) {
     LpOut o{};
-    o.drops = drops;
+    o.drops = cs.flag[F_DROPS];
     o.fail = fail;
     o.warm_used = warm_used == 1 ? 1 : 0;
     if (status == SOV_OPTIMAL) {
       o.status = SOV_OPTIMAL;
       o.iterations = iters;
       o.use_best = 0;
-      o.gap = last_gap;
-      o.p_res = last_p;
-      o.d_res = last_d;
+      o.gap = cs.v[S_GAP];
+      o.p_res = cs.v[S_PRES];
+      o.d_res = cs.v[S_DRES];
     } else {
-      o.status = best_p <= mt.ftol ? SOV_FEASIBLE : SOV_NUMERICAL_ERROR;
-      o.iterations = best_it;
+      o.status = cs.v[S_BP] <= mt.ftol ? SOV_FEASIBLE : SOV_NUMERICAL_ERROR;
+      o.iterations = cs.flag[F_BEST_IT];
       o.use_best = 1;
       o.best_it = status == -2 ? 1 : 0;  // 1: stopped on a failed factorization
-      o.gap = best_gap;
-      o.p_res = best_p;
-      o.d_res = best_d;
+      o.gap = cs.v[S_BGAP];
+      o.p_res = cs.v[S_BP];
+      o.d_res = cs.v[S_BD];
     }
-    o.cx = last_cx;
+    o.cx = cs.v[S_CX];
     bd.out[lp] = o;
   }
   __syncthreads();
@@ -1472,7 +1669,31 @@ int pinned_threads(int mmax) {
   return 0;
 }
 
-int threads_for(int mmax) {
+int sm_count() {
+  int dev = 0, sms = 0;
+  SOV_CUDA(cudaGetDevice(&dev));
+  SOV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  return sms;
+}
+
+// Width of a bucket's CTAs by the LPs of the batch and their mean columns, where no pin and no
+// autotuned choice says otherwise. While every LP has an SM to itself the widest CTA is fastest
+// (its column and row passes scale, the factor's pivot chain does not: 24 transportation LPs 2.16 ms
+// at 128 threads, 1.46 at 256, 1.07 at 512); up to two LPs an SM, 512 threads only for LPs with many
+// columns (300 transportation LPs 1.98 / 1.85 ms at 256 / 512, 200 nodes of 149 columns 0.61 / 1.10);
+// beyond, the choice is between four LPs of 128 threads on an SM and two of 256: long column passes
+// want the wider (4096 transportation LPs, 1225 columns on average: 17.0 / 13.3 ms at 128 / 256;
+// 1000 of 750 columns 2.8 / 2.5 ms), short ones the more resident LPs (3000 LPs of 324 columns 3.2 /
+// 3.8 ms, 1000 nodes 1.5 / 2.2 ms); up to four LPs an SM the line lies lower (400 LPs of 324 columns
+// 0.90 / 0.73 ms, 400 nodes 0.77 / 1.15 ms).
+int width_for(int total, double mean_cols) {
+  const int sms = sm_count();
+  if (total <= sms) return 512;
+  if (total <= 2 * sms) return mean_cols >= 1000.0 ? 512 : 256;
+  return mean_cols >= (total <= 4 * sms ? 250.0 : 600.0) ? 256 : 128;
+}
+
+int threads_for(int mmax, int total, double mean_cols) {
   // SOVEREIGN_BATCH_THREADS=128|129|256|257|512 pins every bucket to a shape (tests run each one
   // this way; odd codes are the lean shapes)
   if (const char* e = std::getenv("SOVEREIGN_BATCH_THREADS")) {
@@ -1484,8 +1705,7 @@ int threads_for(int mmax) {
   std::lock_guard<std::mutex> g(g_tune_mu);
   auto it = g_tuned_threads.find(mmax);
   if (it != g_tuned_threads.end()) return it->second;
-  (void)mmax;
-  return 128;  // measured best on average without tuning (4 CTAs of 128 per SM)
+  return width_for(total, mean_cols);
 }
 
 void launch_any(const BatchDev& bd, int mmax, int code, int grid, cudaStream_t st) {
@@ -1504,13 +1724,6 @@ int tuned_per_sm(int mmax) {
   std::lock_guard<std::mutex> g(g_tune_mu);
   auto it = g_tuned_per_sm.find(mmax);
   return it != g_tuned_per_sm.end() ? it->second : 0;
-}
-
-int sm_count() {
-  int dev = 0, sms = 0;
-  SOV_CUDA(cudaGetDevice(&dev));
-  SOV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  return sms;
 }
 
 int grid_for(int mmax, int code, int count, int per_sm = -1) {
@@ -1669,8 +1882,8 @@ Batch* batch_create(int count, const sov_model* models, const sov_options* opt_i
     std::sort(ids.begin(), ids.end(), [&](int a1, int a2) { return cost[a1] > cost[a2]; });
     auto bk = std::make_unique<Batch::Bucket>();
     bk->mmax = it->first;
-    bk->threads = threads_for(bk->mmax);
     bk->count = static_cast<int>(ids.size());
+    bk->threads = threads_for(bk->mmax, count, static_cast<double>(nv) / count);
     bk->grid = grid_for(bk->mmax, bk->threads, bk->count);
     order_at.push_back(all_orders.size());
     all_orders.insert(all_orders.end(), ids.begin(), ids.end());
