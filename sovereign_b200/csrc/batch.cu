@@ -39,7 +39,6 @@
 
 namespace sov {
 
-constexpr int kBatchMaxRows = 128;
 constexpr int kWarmGiveUp = 40;  // iterations a supplied start gets before the Mehrotra restart
 
 // offset of row i of a row-packed lower triangle

@@ -9,6 +9,8 @@
 
 namespace sov {
 
+constexpr int kBatchMaxRows = 128;  // IPM rows of an LP the batched kernel takes
+
 struct Batch;
 
 // Starts already on the device for every LP of a call (a warm-start network's output): LP k's

@@ -5,7 +5,7 @@ import pytest
 
 import oracle
 from sovereign_b200 import problems as P
-from sovereign_b200.ipm import solve_batch
+from sovereign_b200.ipm import InteriorPointOptions, InteriorPointSolver, solve_batch
 
 pytestmark = pytest.mark.gpu
 
@@ -45,3 +45,62 @@ def test_orders_match_oracle(width, monkeypatch):
         assert r.status_name == ref.status_name == "OPTIMAL", (mdl.name, r.message, ref.message)
         # both stop at a relative gap of 1e-9
         assert abs(r.objective_value - ref.objective_value) <= 1e-8 * max(1.0, abs(ref.objective_value)), mdl.name
+
+
+def both_routes(mdl, monkeypatch, warm=None, **options):
+    """sov_lp_solve by size (one CTA) and through the general engine (a factorization asked for)."""
+    solver = InteriorPointSolver(InteriorPointOptions(**options))
+    auto = solver.solve(mdl, with_ipm=True, warm_start=warm)
+    monkeypatch.setenv("SOVEREIGN_IPM_NORMAL_EQUATIONS", "dense")
+    general = InteriorPointSolver(InteriorPointOptions(**options)).solve(mdl, with_ipm=True, warm_start=warm)
+    monkeypatch.delenv("SOVEREIGN_IPM_NORMAL_EQUATIONS")
+    return auto, general
+
+
+def scaled_bounds(mdl):
+    """Nonzero lower bounds and finite upper bounds on some columns (bound rows), a constant, maximize."""
+    mdl.lb = np.where(np.arange(mdl.n) % 4 == 0, 0.05, 0.0)
+    mdl.ub = np.where(np.arange(mdl.n) % 3 == 0, 300.0, P.INF)
+    mdl.obj, mdl.maximize, mdl.obj_constant = -mdl.obj, True, 2.5
+    return mdl
+
+
+@pytest.mark.parametrize("make,batched", [
+    (lambda: P.bounded_lp_example(), False),                       # two rows share two columns
+    (lambda: P.transport(5, 6, 1), True),
+    (lambda: P.transport(64, 64, 2), True),
+    (lambda: P.transport(64, 65, 2), False),                       # 129 rows
+    (lambda: scaled_bounds(P.transport(8, 9, 5)), True),           # 17 + 24 IPM rows
+    (lambda: scaled_bounds(P.transport(20, 20, 6)), False),        # 40 + 134 IPM rows
+    (lambda: scaled_bounds(P.random_sparse_lp(30, 90, 4, 5)), False),
+    (lambda: P.random_sparse_lp(100, 300, 1, 7), True),            # no off-diagonal entries at all
+])
+def test_single_solve_routes_agree(make, batched, monkeypatch):
+    auto, general = both_routes(make(), monkeypatch)
+    assert ("batched" in auto.message) == batched and "dense Cholesky" in general.message
+    assert auto.status_name == general.status_name == "OPTIMAL"
+    assert auto.iterations == general.iterations and (auto.n_ipm, auto.m_ipm) == (general.n_ipm, general.m_ipm)
+    # the same iteration in another order of summation: within the stopping tolerance of 1e-9
+    assert abs(auto.objective_value - general.objective_value) <= 1e-9 * max(1.0, abs(general.objective_value))
+    assert np.linalg.norm(auto.primal - general.primal) <= 1e-8 * max(1.0, np.linalg.norm(general.primal))
+    assert np.linalg.norm(auto.ipm_x - general.ipm_x) <= 1e-8 * max(1.0, np.linalg.norm(general.ipm_x))
+
+
+def test_single_solve_routes_agree_when_stopped_early_or_warm_started(monkeypatch):
+    mdl = P.transport(9, 11, 4)
+    auto, general = both_routes(mdl, monkeypatch, max_iterations=4)
+    assert auto.status_name == general.status_name != "OPTIMAL"
+    assert auto.iterations == general.iterations and auto.message == general.message
+    start = InteriorPointSolver(InteriorPointOptions(ipm_iterate_at=6)).solve(mdl, with_ipm=True)
+    assert "batched" not in start.message  # an iterate on the way: the general engine
+    auto, general = both_routes(mdl, monkeypatch, warm=(start.ipm_x, start.ipm_y, start.ipm_s))
+    assert "batched" in auto.message and auto.status_name == general.status_name == "OPTIMAL"
+    assert auto.iterations == general.iterations < InteriorPointSolver().solve(mdl).iterations
+    # two calls give the same bits
+    first, second = (InteriorPointSolver().solve(P.transport(31, 29, 8)) for _ in range(2))
+    assert first.objective_value == second.objective_value and np.array_equal(first.primal, second.primal)
+    # infeasible bounds are refused with the general path's message
+    bad = P.transport(3, 3, 1)
+    bad.lb, bad.ub = np.full(9, 2.0), np.full(9, 1.0)
+    auto, general = both_routes(bad, monkeypatch)
+    assert auto.status_name == general.status_name and auto.message == general.message
