@@ -876,7 +876,7 @@ int Family::run() {
 
 void Family::setup_shared(const StdForm& f) {
   // the normal matrices' pattern, its order and symbolic factor, once for the family
-  if (!sparse_analyze(f, 0, sym_))
+  if (!sparse_analyze(f, 0, sym_, SparseOrder::kAuto, false))
     throw std::invalid_argument("sov_lp_solve_family: the sparse L D L' of the order-" + std::to_string(f.m) +
                                 " normal matrix needs more than " + std::to_string(kMaxUpdates) +
                                 " rank-1 update terms");
@@ -884,6 +884,7 @@ void Family::setup_shared(const StdForm& f) {
   // before it -- is factored and solved densely when that costs less than scheduling its terms;
   // one thread per (piece, LP): long items are cut into short pieces
   tail_ = sparse_dense_block(sym_, kSparseTermCost, kMinTail);
+  sparse_updates(sym_, f.m - tail_);
   const SparseSchedule S = sparse_schedule(sym_, tail_, kFamPiece);
   {
     const int T = tail_, mt = f.m - T;

@@ -453,8 +453,8 @@ int sparse_slot(const SparseSymbolic& s, int i, int j) {
   return p < 0 ? -1 : s.m + p;
 }
 
-bool sparse_analyze(const StdForm& f, std::size_t fill_limit, SparseSymbolic& s, SparseOrder order) {
-  if (!sparse_analyze_graph(normal_graph(f), fill_limit, s, order)) return false;
+bool sparse_analyze(const StdForm& f, std::size_t fill_limit, SparseSymbolic& s, SparseOrder order, bool updates) {
+  if (!sparse_analyze_graph(normal_graph(f), fill_limit, s, order, updates)) return false;
   const int m = f.m;
   // assembly map into [D | L]: A's column j couples rows p >= q with weight a_p a_q
   struct Contrib {
@@ -550,7 +550,7 @@ double factor_cost(const Patterns& P) { return (P.hmax + 1) * 5e-6 + P.flops * 1
 }  // namespace
 
 bool sparse_analyze_graph(const std::vector<std::vector<int>>& adj0, std::size_t fill_limit, SparseSymbolic& s,
-                          SparseOrder order) {
+                          SparseOrder order, bool updates) {
   const int m = static_cast<int>(adj0.size());
   s = SparseSymbolic{};
   s.m = m;
@@ -599,29 +599,49 @@ bool sparse_analyze_graph(const std::vector<std::vector<int>>& adj0, std::size_t
     std::vector<int> fill(s.lvl_ptr.begin(), s.lvl_ptr.end() - 1);
     for (int k = 0; k < m; ++k) s.lvl_col[fill[height[k]]++] = k;
   }
+  if (updates) sparse_updates(s, m);
+  return true;
+}
+
+void sparse_updates(SparseSymbolic& s, int before) {
+  const int m = s.m, hmax = s.levels() - 1;
   // rank-1 updates per level, column by column in level order; each column's block of updates is
   // sized up front, so the blocks are filled on several host threads
   std::vector<std::size_t> at(m + 1, 0);
   for (int q = 0; q < m; ++q) {
-    const std::size_t nk = static_cast<std::size_t>(s.lp[s.lvl_col[q] + 1] - s.lp[s.lvl_col[q]]);
+    const int k = s.lvl_col[q];
+    const std::size_t nk = k < before ? static_cast<std::size_t>(s.lp[k + 1] - s.lp[k]) : 0;
     at[q + 1] = at[q] + nk * (nk + 1) / 2;
   }
   s.pairs.resize(4 * at[m]);
   s.pair_ptr.assign(hmax + 2, 0);
   for (int h = 0; h <= hmax; ++h) s.pair_ptr[h + 1] = static_cast<int>(at[s.lvl_ptr[h + 1]]);
+  // Entry (a, b) of column k's block goes to row li[a] of column li[b]. The rows of k below li[b] are
+  // rows of column li[b] too, both lists ascend, so one walk along column li[b] finds all of b's places
+  // (a binary search per entry took most of the analysis of a large factor).
   auto fill_columns = [&](int q0, int q1) {
     for (int q = q0; q < q1; ++q) {
       const int k = s.lvl_col[q];
-      int* out = s.pairs.data() + 4 * at[q];
-      for (int a = s.lp[k]; a < s.lp[k + 1]; ++a)
-        for (int b = s.lp[k]; b <= a; ++b) {
-          const int ia = s.li[a], ib = s.li[b];
+      if (k >= before) continue;
+      int* block = s.pairs.data() + 4 * at[q];
+      const int l0 = s.lp[k], l1 = s.lp[k + 1];
+      for (int b = l0; b < l1; ++b) {
+        const int ib = s.li[b];
+        int pos = s.lp[ib];
+        for (int a = b; a < l1; ++a) {
+          const std::size_t ra = static_cast<std::size_t>(a - l0);
+          int* out = block + 4 * (ra * (ra + 1) / 2 + static_cast<std::size_t>(b - l0));
           out[0] = k;
           out[1] = a;
           out[2] = b;
-          out[3] = ia == ib ? ia : m + position(s, ib, ia);
-          out += 4;
+          if (a == b) {
+            out[3] = ib;
+          } else {
+            while (s.li[pos] != s.li[a]) ++pos;
+            out[3] = m + pos;
+          }
         }
+      }
     }
   };
   const int nthreads = at[m] > 1000000 ? std::max(1, std::min(16, static_cast<int>(std::thread::hardware_concurrency()))) : 1;
@@ -640,7 +660,6 @@ bool sparse_analyze_graph(const std::vector<std::vector<int>>& adj0, std::size_t
     }
     for (std::thread& th : pool) th.join();
   }
-  return true;
 }
 
 namespace {
@@ -730,44 +749,37 @@ SparseSchedule sparse_schedule(const SparseSymbolic& s, int tail, int piece) {
   // column's own updates are left to the dense factorization
   const size_t n_all = s.pairs.size() / 4;
   const int n_dst = m + static_cast<int>(s.li.size());
-  std::vector<int> level_of(n_all);
-  for (int h = 0; h < levels; ++h)
-    for (int u = s.pair_ptr[h]; u < s.pair_ptr[h + 1]; ++u) level_of[u] = h;
-  std::vector<int> keep;
-  keep.reserve(n_all);
+  // pairs lie level by level already: by destination first, then dealt to their levels, each term read
+  // once in destination order (its four numbers share a cache line) and written in place
+  std::vector<size_t> cnt(n_dst + 1, 0), lc(levels + 1, 0);
   for (size_t u = 0; u < n_all; ++u)
-    if (s.pairs[4 * u] < mt) keep.push_back(static_cast<int>(u));
-  const size_t n_up = keep.size();
-  std::vector<int> by_dst(n_up), order(n_up);
-  {
-    std::vector<size_t> cnt(n_dst + 1, 0);
-    for (int u : keep) cnt[s.pairs[4 * u + 3] + 1]++;
-    for (int d = 0; d < n_dst; ++d) cnt[d + 1] += cnt[d];
-    for (int u : keep) by_dst[cnt[s.pairs[4 * u + 3]]++] = u;
-    std::vector<size_t> lc(levels + 1, 0);
-    for (int u : keep) lc[level_of[u] + 1]++;
-    for (int h = 0; h < levels; ++h) lc[h + 1] += lc[h];
-    for (size_t q = 0; q < n_up; ++q) {
-      const int u = by_dst[q];
-      order[lc[level_of[u]]++] = u;
+    if (s.pairs[4 * u] < mt) {
+      cnt[s.pairs[4 * u + 3] + 1]++;
+      lc[level[s.pairs[4 * u]] + 1]++;
     }
-  }
+  for (int d = 0; d < n_dst; ++d) cnt[d + 1] += cnt[d];
+  for (int h = 0; h < levels; ++h) lc[h + 1] += lc[h];
+  const size_t n_up = lc[levels];
+  std::vector<int> by_dst(n_up), dst(n_up);
+  for (size_t u = 0; u < n_all; ++u)
+    if (s.pairs[4 * u] < mt) by_dst[cnt[s.pairs[4 * u + 3]]++] = static_cast<int>(u);
   S.up_col.resize(n_up);
   S.up_a.resize(n_up);
   S.up_b.resize(n_up);
+  std::vector<size_t> fill_at(lc.begin(), lc.end() - 1);
   for (size_t q = 0; q < n_up; ++q) {
-    const int u = order[q];
-    S.up_col[q] = s.pairs[4 * u];
-    S.up_a[q] = s.pairs[4 * u + 1];
-    S.up_b[q] = s.pairs[4 * u + 2];
+    const int* pr = &s.pairs[4 * static_cast<size_t>(by_dst[q])];
+    const size_t o = fill_at[level[pr[0]]]++;
+    S.up_col[o] = pr[0];
+    S.up_a[o] = pr[1];
+    S.up_b[o] = pr[2];
+    dst[o] = pr[3];
   }
-  size_t q = 0;
   for (int h = 0; h < hn; ++h) {
-    while (q < n_up && level_of[order[q]] == h) {
-      const int dst = s.pairs[4 * order[q] + 3];
+    for (size_t q = lc[h]; q < lc[h + 1];) {
       size_t e = q + 1;
-      while (e < n_up && level_of[order[e]] == h && s.pairs[4 * order[e] + 3] == dst) ++e;
-      add_item(S.factor, static_cast<int>(q), static_cast<int>(e), dst, &S.factor_slots, false, piece);
+      while (e < lc[h + 1] && dst[e] == dst[q]) ++e;
+      add_item(S.factor, static_cast<int>(q), static_cast<int>(e), dst[q], &S.factor_slots, false, piece);
       q = e;
     }
     close_level(S.factor);

@@ -47,12 +47,17 @@ constexpr double kMaxUpdates = 2e8;
 // Returns false when the predicted fill exceeds fill_limit entries (0 = no limit) or the update
 // schedule would exceed kMaxUpdates terms.
 bool sparse_analyze(const StdForm& f, std::size_t fill_limit, SparseSymbolic& out,
-                    SparseOrder order = SparseOrder::kAuto);
+                    SparseOrder order = SparseOrder::kAuto, bool updates = true);
+
+// The rank-1 updates (pair_ptr, pairs) of the columns before `before`. The analysis calls it for all
+// columns unless its `updates` is false: a caller that factors a trailing block densely asks for the
+// columns before it alone (a multicommodity family of order 1800: 0.95M of 15M terms).
+void sparse_updates(SparseSymbolic& s, int before);
 
 // The same analysis for any symmetric pattern (adjacency lists without the diagonal, both
 // directions), without an assembly map: the caller places its values with sparse_slot.
 bool sparse_analyze_graph(const std::vector<std::vector<int>>& adj, std::size_t fill_limit, SparseSymbolic& out,
-                          SparseOrder order = SparseOrder::kAuto);
+                          SparseOrder order = SparseOrder::kAuto, bool updates = true);
 
 // Index into the [D | L] value storage of entry (i, j) of the original ordering (-1 if it is not
 // in the pattern of L).
