@@ -106,14 +106,16 @@ __device__ void cta_partials(const FamDev& d, double (&v)[NV], const int (&ops)[
   }
 }
 
-// the blocks' partials of slot q for LP k, in block order
-__device__ __forceinline__ double fold(const FamDev& d, int blocks, int q, int k, int op, double init) {
+// the blocks' partials of slot q for LP k, by one warp: lane l takes blocks l, l + 32, ..., the lanes'
+// results meet in a fixed tree (one thread in block order took 62 us per pass of 296 blocks, a chain of
+// loads; 34 passes of 12 and 18 of 127 us an average family call)
+__device__ __forceinline__ double fold(const FamDev& d, const double* part, int blocks, int q, int k, int op, double init) {
   double acc = init;
-  for (int b = 0; b < blocks; ++b) {
-    const double u = d.part[(static_cast<size_t>(b) * kNv + q) * d.W + k];
+  for (int b = threadIdx.x; b < blocks; b += 32) {
+    const double u = part[(static_cast<size_t>(b) * kNv + q) * d.W + k];
     acc = op == 0 ? acc + u : op == 1 ? fmax(acc, u) : fmin(acc, u);
   }
-  return acc;
+  return op == 0 ? warp_sum(acc) : op == 1 ? warp_max(acc) : warp_min(acc);
 }
 
 // ---- residuals: rp = b - A x, rd = c - (A'y + s) (interior_point.cpp:572-602) ----
@@ -154,15 +156,14 @@ __global__ void k_fam_res_cols(FamDev d) {
   cta_partials<3>(d, v, ops, sm);
 }
 
-// one thread per LP: rows' and columns' partials (two part buffers) into the scalars
+// one warp per LP: rows' and columns' partials (two part buffers) into the scalars
 __global__ void k_fam_res_final(FamDev d, const double* rows_part, int rows_blocks, int cols_blocks) {
-  const int k = threadIdx.x;
-  if (k >= d.W) return;
-  double rpm = 0.0;
-  for (int b = 0; b < rows_blocks; ++b) rpm = fmax(rpm, rows_part[(static_cast<size_t>(b) * kNv) * d.W + k]);
-  const double rdm = fold(d, cols_blocks, 0, k, 1, 0.0);
-  const double xs = fold(d, cols_blocks, 1, k, 0, 0.0);
-  const double cx = fold(d, cols_blocks, 2, k, 0, 0.0);
+  const int k = blockIdx.x;
+  const double rpm = fold(d, rows_part, rows_blocks, 0, k, 1, 0.0);
+  const double rdm = fold(d, d.part, cols_blocks, 0, k, 1, 0.0);
+  const double xs = fold(d, d.part, cols_blocks, 1, k, 0, 0.0);
+  const double cx = fold(d, d.part, cols_blocks, 2, k, 0, 0.0);
+  if (threadIdx.x != 0) return;
   FamScalars& sc = d.sc[k];
   sc.rp_max = rpm;
   sc.rd_max = rdm;
@@ -233,9 +234,9 @@ __global__ void k_fam_direction(FamDev d, int mode) {
 }
 
 __global__ void k_fam_direction_final(FamDev d, int mode, int blocks) {
-  const int k = threadIdx.x;
-  if (k >= d.W) return;
-  const double rp = fold(d, blocks, 0, k, 2, 1.0), rdd = fold(d, blocks, 1, k, 2, 1.0);
+  const int k = blockIdx.x;
+  const double rp = fold(d, d.part, blocks, 0, k, 2, 1.0), rdd = fold(d, d.part, blocks, 1, k, 2, 1.0);
+  if (threadIdx.x != 0) return;
   FamScalars& sc = d.sc[k];
   sc.ratio_p = rp;
   sc.ratio_d = rdd;
@@ -264,10 +265,11 @@ __global__ void k_fam_mu_aff(FamDev d) {
 }
 
 __global__ void k_fam_mu_final(FamDev d, int blocks) {
-  const int k = threadIdx.x;
-  if (k >= d.W) return;
+  const int k = blockIdx.x;
+  const double total = fold(d, d.part, blocks, 0, k, 0, 0.0);
+  if (threadIdx.x != 0) return;
   FamScalars& sc = d.sc[k];
-  sc.mu_aff = fold(d, blocks, 0, k, 0, 0.0) / static_cast<double>(d.n);
+  sc.mu_aff = total / static_cast<double>(d.n);
   const double r = sc.mu_aff / sc.mu;
   sc.sigma = sc.mu > 0.0 ? fmin(1.0, r * r * r) : 0.0;
 }
@@ -689,6 +691,153 @@ __global__ void __launch_bounds__(kFamThreads) k_fam_solve(FamSparse f, double* 
   for (long long t = rank; t < mw; t += size) z[static_cast<size_t>(f.perm[t / W]) * W + t % W] = f.work[t];
 }
 
+// The same solve with a CTA per LP, the right-hand side and 1 / D in shared memory: LPs do not depend on
+// one another, so nothing needs a grid barrier (k_fam_solve takes about 130 of them, some 5 us each, and
+// a dependent L2 load per step of a panel's triangle). One LP's values are 8 of every 32-byte sector read,
+// which L2 bears: the factor's 128000 entries are 4 MB of sectors an LP. Loads of a piece, of a panel's
+// triangle and of a row's panel terms are issued together; the triangles are the last warp's, whose loads
+// for the next panel overlap the rows' update. Same pieces, same order of every sum: bit-identical to
+// k_fam_solve. Measured (64 multicommodity LPs of order 1800, 456 tail columns): 1.70 -> 0.42 ms a solve.
+constexpr int kLpThreads = 512;
+
+// sum of `count` terms in order, eight terms' loads ahead of their products
+template <class Load, class Product>
+__device__ __forceinline__ double ahead_sum(int count, Load load, Product product) {
+  double acc = 0.0;
+  int q = 0;
+  for (; q + 8 <= count; q += 8) {
+    double v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = load(q + e);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc += product(q + e, v[e]);
+  }
+  if (q < count) {
+    double v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = q + e < count ? load(q + e) : 0.0;
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (q + e < count) acc += product(q + e, v[e]);
+  }
+  return acc;
+}
+
+__global__ void __launch_bounds__(kLpThreads) k_fam_solve_lp(FamSparse f, double* z) {
+  extern __shared__ double fam_sm[];
+  const int W = f.W, lp = blockIdx.x, m = f.m;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double* work = fam_sm;
+  double* inv = fam_sm + m;
+  for (int t = tid; t < m; t += kLpThreads) {
+    work[t] = z[static_cast<size_t>(f.perm[t]) * W + lp];
+    inv[t] = f.inv_d[static_cast<size_t>(t) * W + lp];
+  }
+  __syncthreads();
+  auto v_at = [&](int pos) { return f.V[static_cast<size_t>(m + pos) * W + lp]; };
+  auto combine = [&](const int4* combs, int c0, int c1, auto apply) {
+    if (c1 <= c0) return;  // uniform over the CTA
+    __syncthreads();
+    for (int c = c0 + tid; c < c1; c += kLpThreads) {
+      const int4 cb = combs[c];
+      double acc = 0.0;
+      for (int q = 0; q < cb.z; ++q) acc += f.partial[static_cast<size_t>(cb.y + q) * W + lp];
+      apply(cb.x, acc);
+    }
+  };
+  const int fwd_levels = f.levels + (f.tail > 0 ? 1 : 0);  // + the tail rows' sums before the tail
+  for (int h = 0; h < fwd_levels; ++h) {
+    for (int q = f.lpiece_lvl[h] + tid; q < f.lpiece_lvl[h + 1]; q += kLpThreads) {
+      const int4 pc = f.lpiece[q];
+      const double acc = ahead_sum(
+          pc.y - pc.x, [&](int e) { return v_at(f.row_pos[pc.x + e]); },
+          [&](int e, double v) {
+            const int c = f.row_col[pc.x + e];
+            return v * inv[c] * work[c];
+          });
+      if (pc.w < 0) work[pc.z] -= acc;
+      else f.partial[static_cast<size_t>(pc.w) * W + lp] = acc;
+    }
+    combine(f.lcomb, f.lcomb_lvl[h], f.lcomb_lvl[h + 1], [&](int x, double acc) { work[x] -= acc; });
+    __syncthreads();
+  }
+  if (f.tail > 0) {
+    const int T = f.tail, mt = f.mt;
+    const bool triangle = warp == kLpThreads / 32 - 1;
+    double l[kSolvePanel];
+    auto load_forward = [&](int j0) {  // row j0 + lane of the panel's triangle
+#pragma unroll
+      for (int j = 0; j < kSolvePanel; ++j)
+        l[j] = lane > j && j0 + lane < T ? f.Ld[tail_at(f, j0 + lane, j0 + j, lp)] : 0.0;
+    };
+    if (triangle) load_forward(0);
+    for (int j0 = 0; j0 < T; j0 += kSolvePanel) {
+      const int P = min(T, j0 + kSolvePanel) - j0, j1 = j0 + P;
+      if (triangle) {
+        const bool on = lane < P;
+        double y = on ? work[mt + j0 + lane] : 0.0;
+        const double d = on ? inv[mt + j0 + lane] : 0.0;
+#pragma unroll
+        for (int j = 0; j < kSolvePanel; ++j) {
+          const double coef = __shfl_sync(kFull, y * d, j);
+          if (on && lane > j) y -= l[j] * coef;
+        }
+        if (on) work[mt + j0 + lane] = y;
+        if (j1 < T) load_forward(j1);
+      }
+      __syncthreads();
+      for (int a = j1 + tid; a < T; a += kLpThreads)
+        work[mt + a] -= ahead_sum(
+            P, [&](int e) { return f.Ld[tail_at(f, a, j0 + e, lp)]; },
+            [&](int e, double v) { return v * work[mt + j0 + e] * inv[mt + j0 + e]; });
+      __syncthreads();
+    }
+    const int last = (T - 1) / kSolvePanel * kSolvePanel;
+    auto load_backward = [&](int j0) {  // column j0 + lane of the panel's triangle
+#pragma unroll
+      for (int i = 0; i < kSolvePanel; ++i)
+        l[i] = lane < i && j0 + i < T ? f.Ld[tail_at(f, j0 + i, j0 + lane, lp)] : 0.0;
+    };
+    if (triangle) load_backward(last);
+    for (int j0 = last; j0 >= 0; j0 -= kSolvePanel) {
+      const int P = min(T, j0 + kSolvePanel) - j0;
+      if (triangle) {
+        const bool on = lane < P;
+        double y = on ? work[mt + j0 + lane] : 0.0;
+        const double d = on ? inv[mt + j0 + lane] : 0.0;
+#pragma unroll
+        for (int i = kSolvePanel - 1; i >= 0; --i) {
+          const double xi = __shfl_sync(kFull, y * d, i);
+          if (lane == i && i < P) y = xi;
+          if (on && lane < i && i < P) y -= l[i] * xi;
+        }
+        if (on) work[mt + j0 + lane] = y;
+        if (j0 > 0) load_backward(j0 - kSolvePanel);
+      }
+      __syncthreads();
+      for (int k = tid; k < j0; k += kLpThreads)
+        work[mt + k] -= ahead_sum(
+            P, [&](int e) { return f.Ld[tail_at(f, j0 + e, k, lp)]; },
+            [&](int e, double v) { return v * work[mt + j0 + e]; });
+      __syncthreads();
+    }
+  }
+  for (int h = f.levels - 1; h >= 0; --h) {
+    for (int q = f.upiece_lvl[h] + tid; q < f.upiece_lvl[h + 1]; q += kLpThreads) {
+      const int4 pc = f.upiece[q];
+      const double acc = ahead_sum(
+          pc.y - pc.x, [&](int e) { return v_at(pc.x + e); },
+          [&](int e, double v) { return v * work[f.li[pc.x + e]]; });
+      if (pc.w < 0) work[pc.z] = (work[pc.z] - acc) * inv[pc.z];
+      else f.partial[static_cast<size_t>(pc.w) * W + lp] = acc;
+    }
+    combine(f.ucomb, f.ucomb_lvl[h], f.ucomb_lvl[h + 1],
+            [&](int x, double acc) { work[x] = (work[x] - acc) * inv[x]; });
+    __syncthreads();
+  }
+  for (int t = tid; t < m; t += kLpThreads) z[static_cast<size_t>(f.perm[t]) * W + lp] = work[t];
+}
+
 // ---------------------------------------------------------------------------------------------
 // host side
 
@@ -780,6 +929,7 @@ class Family {
   std::vector<sov_options> opts_;
   std::vector<StdForm> forms_;
   cudaStream_t st_ = nullptr;
+  size_t smem_max_ = 0;
   int sms_ = 148, per_sm_factor_ = 1, per_sm_solve_ = 1;
   // shared structure
   SparseSymbolic sym_;
@@ -961,6 +1111,12 @@ void Family::setup_shared(const StdForm& f) {
   int dev = 0;
   SOV_CUDA(cudaGetDevice(&dev));
   SOV_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
+  int smem_max = 0;
+  SOV_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  smem_max_ = static_cast<size_t>(smem_max);
+  once_per_device((const void*)k_fam_solve_lp, [&] {
+    SOV_CUDA(cudaFuncSetAttribute(k_fam_solve_lp, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
+  });
   SOV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_factor_, k_fam_factor, kFamThreads, 0));
   SOV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_solve_, k_fam_solve, kFamThreads, 0));
   per_sm_factor_ = std::max(1, std::min(per_sm_factor_, 2));
@@ -1041,7 +1197,7 @@ void Family::residuals() {
   const int gr = grid_for(dev_.m), gc = grid_for(dev_.n);
   k_fam_res_rows<<<gr, bd, smem, st_>>>(rows);
   k_fam_res_cols<<<gc, bd, smem, st_>>>(dev_);
-  k_fam_res_final<<<1, kFamilyWidth, 0, st_>>>(dev_, part_rows_.p, gr, gc);
+  k_fam_res_final<<<dev_.W, 32, 0, st_>>>(dev_, part_rows_.p, gr, gc);
   SOV_LAUNCH_CHECK();
 }
 
@@ -1079,6 +1235,13 @@ void Family::factor() {
 
 void Family::solve(double* z) {
   FamSparse f = sp_;
+  // a CTA per LP while an LP's two vectors fit in shared memory (order 12000 and more do)
+  const size_t smem = 2 * sizeof(double) * static_cast<size_t>(f.m);
+  if (smem <= smem_max_) {
+    k_fam_solve_lp<<<f.W, kLpThreads, smem, st_>>>(f, z);
+    SOV_LAUNCH_CHECK();
+    return;
+  }
   void* args[] = {&f, &z};
   SOV_CUDA(cudaLaunchCooperativeKernel((const void*)k_fam_solve, dim3(sms_ * per_sm_solve_), dim3(kFamThreads), args, 0,
                                        st_));
@@ -1495,10 +1658,10 @@ void Family::solve_wave(const std::vector<int>& lps) {
       k_fam_newton_rhs<<<grid_for(m), bd, 0, st_>>>(dev_);
       solve(z_.p);
       k_fam_direction<<<gn, bd, smem, st_>>>(dev_, pass);
-      k_fam_direction_final<<<1, kFamilyWidth, 0, st_>>>(dev_, pass, gn);
+      k_fam_direction_final<<<W, 32, 0, st_>>>(dev_, pass, gn);
       if (pass == 0) {
         k_fam_mu_aff<<<gn, bd, smem, st_>>>(dev_);
-        k_fam_mu_final<<<1, kFamilyWidth, 0, st_>>>(dev_, gn);
+        k_fam_mu_final<<<W, 32, 0, st_>>>(dev_, gn);
       }
     }
     k_fam_update<<<grid_for(std::max(n, m)), bd, 0, st_>>>(dev_);
