@@ -4,13 +4,17 @@
 //
 // One 128 x 128 output tile per CTA (all tiles, or those on or below the diagonal). Operands are FP32 in global
 // memory with arbitrary row / K strides; they stream through kStages shared-memory stages in K
-// chunks. Warps 0-3 are producers: each thread converts its 16-byte groups of a chunk (coalesced
-// along whichever operand dimension is contiguous) to the tensor-core type and stores them in the
+// chunks. Warps 0-7 are producers: each thread converts its 16-byte groups of a chunk (coalesced
+// along whichever operand dimension is contiguous, in 16-byte loads where K is contiguous and the
+// rows are 16-byte aligned) to the tensor-core type and stores them in the
 // canonical K-major no-swizzle layout (8-row x 16-byte core matrices; LBO 128 B, SBO 1024 B), then
-// arrives on the stage's "full" barrier. Lane 0 of warp 4 issues tcgen05.mma from the stage into a
+// arrives on the stage's "full" barrier. Lane 0 of warp 8 issues tcgen05.mma from the stage into a
 // TMEM accumulator (128 lanes x 128 FP32 columns) and commits the stage's "empty" barrier, so
 // loading chunk k + kStages - 1 overlaps the MMAs of chunk k. After the last chunk the MMA thread
-// commits "done" and warps 0-3 read the accumulator back with tcgen05.ld for the epilogue.
+// commits "done" and warps 0-7 read the accumulator back with tcgen05.ld for the epilogue.
+// With few output tiles the producers bound it: one SM reads 64 KB a BF16 chunk, and the loads in flight
+// set the rate, hence eight warps of them rather than four, wide loads and conflict-free stores (gradient of a 4040-512-512-512-11800
+// network, 256 rows: 2.0 -> 0.9 ms in its eleven products; a 640-wide 3xTF32 update 20 -> 14 us).
 //   KIND 1: BF16 operands (kind::f16, K = 16 per MMA), 64-wide K chunks, 4 stages (128 KB).
 //   KIND 0: 3xTF32 (kind::tf32, K = 8 per MMA): each FP32 operand split into hi = tf32(a) and
 //           lo = tf32(a - hi); a_hi b_hi + a_hi b_lo + a_lo b_hi accumulate in FP32, close to FP32
@@ -46,7 +50,8 @@ struct WsGemmArgs {
 namespace wsg {
 
 constexpr int kTile = 128;
-constexpr int kThreads = 160;       // warps 0-3: producers and epilogue; warp 4: MMA issue
+constexpr int kProducers = 256;
+constexpr int kThreads = kProducers + 32;  // warps 0-7: producers and epilogue; warp 8: MMA issue
 constexpr int kOperandBytes = 16384;  // 128 rows x 128 bytes of K
 constexpr long long kWaitLimit = 1ll << 22;  // try_wait polls: a few seconds at most
 
@@ -76,39 +81,62 @@ __device__ __forceinline__ float to_tf32(float v) {
   return __uint_as_float(r);
 }
 
-// Stage one operand's chunk: rows [row0, row0 + 128) x K [k0, k0 + kK) of X, 8 groups per thread.
+// Stage one operand's chunk: rows [row0, row0 + 128) x K [k0, k0 + kK) of X, 4 groups per thread.
 template <int KIND>
 __device__ __forceinline__ void stage_operand(const float* X, long long rs, long long ks, int row0, int rows, int k0,
                                               int K, unsigned char* hi, unsigned char* lo, int p) {
   using C = Cfg<KIND>;
   constexpr int kGroupsPerRow = C::kK / C::kGroup;  // 8
-  constexpr int kPer = kTile * kGroupsPerRow / 128;  // groups per producer thread: 8
+  constexpr int kPer = kTile * kGroupsPerRow / kProducers;  // groups per producer thread: 4
+  static_assert(kGroupsPerRow == 8, "group order");
   const bool k_contig = ks == 1;
+  // Group g's row and K group. Eight threads in a row take the eight rows of a core matrix, whose
+  // 16-byte groups are the 128 bytes a shared-memory store moves at once (with a row's eight groups on
+  // them instead, stores 128 bytes apart, they all met in the same banks); K contiguous: the four
+  // such octets of a warp are K groups of the same rows, 128 (64) bytes of each; else 32 rows.
+  auto row_of = [&](int g) { return k_contig ? (g >> 6) * 8 + (g & 7) : g % kTile; };
+  auto kg_of = [&](int g) { return k_contig ? (g >> 3) & 7 : g / kTile; };
   // The loads of a batch of groups are all issued before the first shared-memory store: the stores
   // go through generic pointers the compiler cannot tell apart from X, so a load placed after a
   // store would wait for it, and the chunk would cost one global round trip per group.
-  constexpr int kBatch = KIND == 1 ? 4 : 8;  // groups in flight: 32 floats either way
+  constexpr int kBatch = kPer;  // groups in flight
+  // 16-byte loads: K contiguous, every row of X on a 16-byte boundary, the chunk inside K
+  const bool wide = k_contig && (rs & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0 && k0 + C::kK <= K;
 #pragma unroll
   for (int b0 = 0; b0 < kPer; b0 += kBatch) {
     float v[kBatch][C::kGroup];
+    if (wide) {
 #pragma unroll
-    for (int ib = 0; ib < kBatch; ++ib) {
-      const int g = (b0 + ib) * 128 + p;
-      const int row = k_contig ? g / kGroupsPerRow : g % kTile;
-      const int kg = k_contig ? g % kGroupsPerRow : g / kTile;
-      const int gr = row0 + row;
+      for (int ib = 0; ib < kBatch; ++ib) {
+        const int g = (b0 + ib) * kProducers + p;
+        const int gr = row0 + row_of(g);
+        const float4* src = reinterpret_cast<const float4*>(X + gr * rs + k0 + kg_of(g) * C::kGroup);
 #pragma unroll
-      for (int e = 0; e < C::kGroup; ++e) {
-        const int gk = k0 + kg * C::kGroup + e;
-        v[ib][e] = (gr < rows && gk < K) ? X[gr * rs + gk * ks] : 0.0f;
+        for (int e = 0; e < C::kGroup / 4; ++e) {
+          const float4 q = gr < rows ? src[e] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          v[ib][4 * e] = q.x;
+          v[ib][4 * e + 1] = q.y;
+          v[ib][4 * e + 2] = q.z;
+          v[ib][4 * e + 3] = q.w;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int ib = 0; ib < kBatch; ++ib) {
+        const int g = (b0 + ib) * kProducers + p;
+        const int kg = kg_of(g);
+        const int gr = row0 + row_of(g);
+#pragma unroll
+        for (int e = 0; e < C::kGroup; ++e) {
+          const int gk = k0 + kg * C::kGroup + e;
+          v[ib][e] = (gr < rows && gk < K) ? X[gr * rs + gk * ks] : 0.0f;
+        }
       }
     }
 #pragma unroll
     for (int ib = 0; ib < kBatch; ++ib) {
-      const int g = (b0 + ib) * 128 + p;
-      const int row = k_contig ? g / kGroupsPerRow : g % kTile;
-      const int kg = k_contig ? g % kGroupsPerRow : g / kTile;
-      const uint32_t off = tc::kmajor_offset(row, kg * C::kGroup, C::kK, KIND == 1 ? 2 : 4);
+      const int g = (b0 + ib) * kProducers + p;
+      const uint32_t off = tc::kmajor_offset(row_of(g), kg_of(g) * C::kGroup, C::kK, KIND == 1 ? 2 : 4);
       if constexpr (KIND == 1) {
         uint4 w;
         __nv_bfloat162 q0 = __floats2bfloat162_rn(v[ib][0], v[ib][1]), q1 = __floats2bfloat162_rn(v[ib][2], v[ib][3]);
@@ -152,7 +180,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_ws(WsGemmArgs g) {
   if (warp == 0) tc::tmem_alloc(&tmem_base, kTile);
   if (tid == 0) {
     for (int s = 0; s < C::kStages; ++s) {
-      tc::mbar_init(&full[s], 128);
+      tc::mbar_init(&full[s], kProducers);
       tc::mbar_init(&empty[s], 1);
     }
     tc::mbar_init(&done, 1);
@@ -165,7 +193,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_ws(WsGemmArgs g) {
   const uint32_t tmem = tmem_base;
   auto stage_ptr = [&](int s, int operand) { return smem + (static_cast<size_t>(s) * C::kOperands + operand) * kOperandBytes; };
   bool ok = true;
-  if (warp < 4) {
+  if (warp < kProducers / 32) {
     // ---- producers ----
     for (int kc = 0; kc < nk && ok; ++kc) {
       const int s = kc % C::kStages;
@@ -221,22 +249,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_ws(WsGemmArgs g) {
     if (!ok) atomicExch(&s_fail, 1);
   }
   __syncwarp();
-  // ---- epilogue (warps 0-3) ----
+  // ---- epilogue (warps 0-7: warp w reads TMEM lanes 32 (w % 4) .., half of the columns) ----
   bool have = false;
-  if (warp < 4) {
+  if (warp < kProducers / 32) {
     have = tc::mbar_wait(&done, 0, kWaitLimit);
     tc::fence_after();
   }
   __syncwarp();
   __syncthreads();
   const bool fine = have && s_fail == 0;
-  if (warp < 4) {
+  if (warp < kProducers / 32) {
     if (fine) {
-      const int r = r0 + warp * 32 + lane;
+      const int quad = warp & 3, r = r0 + quad * 32 + lane;
 #pragma unroll 1
-      for (int cc = 0; cc < kTile / 32; ++cc) {
+      for (int cc = (warp >> 2) * 2; cc < (warp >> 2) * 2 + 2; ++cc) {
         float v[32];
-        tc::tmem_ld32(tmem + (static_cast<uint32_t>(warp * 32) << 16) + cc * 32, v);
+        tc::tmem_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) + cc * 32, v);
         if (r < g.M) {
           // the 32 old values of C are read before the first store (a read after a store to
           // a possibly aliasing address would wait for it: one round trip per column)
