@@ -20,8 +20,10 @@ struct DenseSystem {
   int m, mp, nb;
   int* drop_count;   // dropped pivots (dependent rows)
   int* fail;         // non-finite pivot
-  unsigned* flags;   // nb: dataflow flags for the factor's panels and the triangular solves
+  unsigned* flags;   // nb: dataflow flags for the factor's panels
   unsigned* tickets; // 1: work-item counter of the factor's panel launches
+  double* chain;     // 2 mp: where the triangular solves publish their blocks; every byte 0xFF before the
+                     // first solve (dense_chain_reset), and left so that the next solve can follow
   double drop_tol;   // pivot <= drop_tol * diag is a dependent row (1e-13 FP64, looser for FP32)
 };
 
@@ -67,8 +69,10 @@ void dense_cholesky_tc(const DenseSystem<float>& s, int* err, cudaStream_t st, i
 
 // In-place solve of L L' z = r for one FP64 right-hand side of length mp (padding entries 0).
 template <class T>
-void dense_solve(const DenseSystem<T>& s, double* z, unsigned& epoch, int* err, cudaStream_t st,
-                 int* launches);
+void dense_solve(const DenseSystem<T>& s, double* z, int* err, cudaStream_t st, int* launches);
+inline void dense_chain_reset(double* chain, int mp, cudaStream_t st) {
+  cudaMemsetAsync(chain, 0xff, 2 * sizeof(double) * static_cast<size_t>(mp), st);
+}
 
 // Y <- L^-1 Y for nrhs columns (column-major, ldy >= mp, padding rows 0). `flags`: dense_forward_flags
 // entries of device memory, cleared by the call; *err is set if a wait gives up.

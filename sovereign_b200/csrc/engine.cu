@@ -263,10 +263,9 @@ class Engine {
   AssemblyDev amd_{};
   DevBuf<double> M64_, Linv64_;
   DevBuf<float> M32_, Linv32_;
-  DevBuf<double> diag_, band_, dinv_;
+  DevBuf<double> diag_, band_, dinv_, chain_, hchain_;
   DevBuf<unsigned> flags_;
   DevBuf<int> err_;
-  unsigned epoch_ = 0;
   DenseSystem<double> ds64_{};
   DenseSystem<float> ds32_{};
   BandSystem bandsys_{};
@@ -445,6 +444,8 @@ void Engine::setup() {
     diag_.alloc(order_);
     flags_.alloc(nb_ + 1);  // + the factor's ticket counter
     flags_.zero(st_);
+    chain_.alloc(2 * static_cast<size_t>(mp_));
+    dense_chain_reset(chain_.p, mp_, st_);
     z_.alloc(mp_);
     z_.zero(st_);
     if (backend_ == kDenseMixed) {
@@ -485,6 +486,8 @@ void Engine::setup() {
     hdiag_.alloc(n);
     hflags_.alloc(nbh_ + 1);
     hflags_.zero(st_);
+    hchain_.alloc(2 * static_cast<size_t>(nph_));
+    dense_chain_reset(hchain_.p, nph_, st_);
     ymat_.alloc(static_cast<size_t>(nph_) * std::max(1, m));
     hfwd_flags_.alloc(dense_forward_flags(nbh_, m));
     hvec_.alloc(nph_);
@@ -521,7 +524,7 @@ void Engine::setup() {
     bandsys_.drop_count = drop_ptr;
     bandsys_.fail = fail_ptr;
   } else {
-    ds32_ = DenseSystem<float>{M32_.p, Linv32_.p, diag_.p, order_, mp_, nb_, drop_ptr, fail_ptr, flags_.p, flags_.p + nb_, 1e-6};
+    ds32_ = DenseSystem<float>{M32_.p, Linv32_.p, diag_.p, order_, mp_, nb_, drop_ptr, fail_ptr, flags_.p, flags_.p + nb_, chain_.p, 1e-6};
   }
   if (backend_ == kKkt) {
     kkt_ = std::make_unique<KktSystem>();
@@ -529,7 +532,7 @@ void Engine::setup() {
                 rval_.p, free_.p, drop_ptr, fail_ptr, st_);
   } else if (coupled_) {
     dsh_ = DenseSystem<double>{hmat_.p, hlinv_.p, hdiag_.p, n, nph_, nbh_, drop_ptr, fail_ptr, hflags_.p,
-                               hflags_.p + nbh_, 1e-13};
+                               hflags_.p + nbh_, hchain_.p, 1e-13};
   }
 
   dev_.m = m;
@@ -644,7 +647,7 @@ void Engine::assemble_and_factor(int mode) {
     if (!M64_.p) {
       M64_.alloc(static_cast<size_t>(mp_) * mp_);
       Linv64_.alloc(static_cast<size_t>(nb_) * kNB * kNB);
-      ds64_ = DenseSystem<double>{M64_.p, Linv64_.p, diag_.p, order_, mp_, nb_, &sc_.p->drops, &sc_.p->fail, flags_.p, flags_.p + nb_, 1e-13};
+      ds64_ = DenseSystem<double>{M64_.p, Linv64_.p, diag_.p, order_, mp_, nb_, &sc_.p->drops, &sc_.p->fail, flags_.p, flags_.p + nb_, chain_.p, 1e-13};
     }
     if (coupled_ && mode != kWeightOnes) {
       // H = Q + diag(h) = L L'; Y = L^-1 A'; M = A H^-1 A' + reg I = Y'Y + reg I, factored (the
@@ -745,11 +748,11 @@ void Engine::coupled_newton(int mode) {
     return;
   }
   launch_hessian_r1(dev_, mode, hvec_.p, st_);
-  dense_solve<double>(dsh_, hvec_.p, epoch_, err_.p, st_, &launches_);
+  dense_solve<double>(dsh_, hvec_.p, err_.p, st_, &launches_);
   launch_rows_minus(dev_, hvec_.p, rp_.p, st_);
   newton_solve();
   launch_hessian_w(dev_, mode, hvec_.p, st_);
-  dense_solve<double>(dsh_, hvec_.p, epoch_, err_.p, st_, &launches_);
+  dense_solve<double>(dsh_, hvec_.p, err_.p, st_, &launches_);
   launch_direction_dx(dev_, mode, hvec_.p, st_, &launches_);
   launches_ += 3;
 }
@@ -769,7 +772,7 @@ bool Engine::newton_solve() {
     return true;
   }
   if (backend_ == kDense64) {
-    dense_solve<double>(ds64_, z_.p, epoch_, err_.p, st_, &launches_);
+    dense_solve<double>(ds64_, z_.p, err_.p, st_, &launches_);
     return true;
   }
   // mixed: PCG on (A D A' + reg I) dy = z with the FP32 factor as preconditioner
@@ -777,7 +780,7 @@ bool Engine::newton_solve() {
   const double reg = 1e-12;
   const double tol2 = 1e-22;  // ||r|| <= 1e-11 ||b||
   k_pcg_init<<<1, 1024, 0, st_>>>(m, z_.p, pcg_x_.p, pcg_r_.p, pcg_w_.p, pcg_s_.p);
-  dense_solve<float>(ds32_, pcg_w_.p, epoch_, err_.p, st_, &launches_);
+  dense_solve<float>(ds32_, pcg_w_.p, err_.p, st_, &launches_);
   k_pcg_direction<<<1, 1024, 0, st_>>>(m, pcg_r_.p, pcg_w_.p, pcg_p_.p, pcg_s_.p, 1);
   launches_ += 2;
   bool converged = false;
@@ -794,7 +797,7 @@ bool Engine::newton_solve() {
       converged = std::isfinite(pcg_h_->rr);
       break;
     }
-    dense_solve<float>(ds32_, pcg_w_.p, epoch_, err_.p, st_, &launches_);
+    dense_solve<float>(ds32_, pcg_w_.p, err_.p, st_, &launches_);
     k_pcg_direction<<<1, 1024, 0, st_>>>(m, pcg_r_.p, pcg_w_.p, pcg_p_.p, pcg_s_.p, 0);
     launches_ += 1;
   }
@@ -809,14 +812,14 @@ bool Engine::newton_solve() {
     if (!M64_.p) {
       M64_.alloc(static_cast<size_t>(mp_) * mp_);
       Linv64_.alloc(static_cast<size_t>(nb_) * kNB * kNB);
-      ds64_ = DenseSystem<double>{M64_.p, Linv64_.p, diag_.p, order_, mp_, nb_, &sc_.p->drops, &sc_.p->fail, flags_.p, flags_.p + nb_, 1e-13};
+      ds64_ = DenseSystem<double>{M64_.p, Linv64_.p, diag_.p, order_, mp_, nb_, &sc_.p->drops, &sc_.p->fail, flags_.p, flags_.p + nb_, chain_.p, 1e-13};
     }
     launch_dense_clear<double>(M64_.p, f_.m, mp_, st_);
     launch_assemble<double>(amd_, x_.p, s_.p, qdiag_.p, free_.p, last_mode_, reg, M64_.p, diag_.p, f_.m, mp_, st_);
     dense_cholesky<double>(ds64_, st_, &launches_);
     fp64_ready_ = true;
   }
-  dense_solve<double>(ds64_, z_.p, epoch_, err_.p, st_, &launches_);
+  dense_solve<double>(ds64_, z_.p, err_.p, st_, &launches_);
   return true;
 }
 

@@ -32,7 +32,7 @@ constexpr int kNoAllocMaxRows = SOV_NOALLOC_MAX_ROWS;  // 512
 constexpr int kNoAllocMaxBlocks = kNoAllocMaxRows / kNB;
 constexpr size_t kScratchM = static_cast<size_t>(kNoAllocMaxRows) * kNoAllocMaxRows;
 constexpr size_t kScratchLinv = static_cast<size_t>(kNoAllocMaxBlocks) * kNB * kNB;
-constexpr size_t kScratchDoubles = kScratchM + kScratchLinv + 2 * kNoAllocMaxRows;
+constexpr size_t kScratchDoubles = kScratchM + kScratchLinv + 4 * kNoAllocMaxRows;  // z, diagonal, 2 x solve chain
 constexpr int kScratchInts = 64 + 8;  // flags (up to 64 blocks) + counters
 
 static __device__ __align__(256) double g_scratch[kScratchDoubles];
@@ -139,12 +139,14 @@ extern "C" int sov_normal_factor_solve_noalloc(int32_t m, int32_t n, const int32
     double* Linv = sp.d + kScratchM;
     double* z = Linv + kScratchLinv;
     double* diag = z + kNoAllocMaxRows;
+    double* chain = diag + kNoAllocMaxRows;
     unsigned* flags = reinterpret_cast<unsigned*>(sp.i);
     // [0] dropped pivots, [1] non-finite pivot, [2] solve timeout, [3] tickets, [4] bad entries
     int* counters = sp.i + 64;
     // clear what must start at zero: the matrix, the flags and the counters
     SOV_CUDA(cudaMemsetAsync(M, 0, sizeof(double) * static_cast<size_t>(mp) * mp, st));
     SOV_CUDA(cudaMemsetAsync(sp.i, 0, sizeof(int) * kScratchInts, st));
+    dense_chain_reset(chain, mp, st);
     if (n > 0) k_scatter_normal<<<ceil_div(n, 128), 128, 0, st>>>(n, m, col_ptr, row_idx, values, d, M, mp, counters + 4);
     SOV_LAUNCH_CHECK();
     int bad = 0;
@@ -156,13 +158,12 @@ extern "C" int sov_normal_factor_solve_noalloc(int32_t m, int32_t n, const int32
     k_finish_diag<<<ceil_div(mp, 128), 128, 0, st>>>(M, m, mp, diag);
     SOV_LAUNCH_CHECK();
     DenseSystem<double> s{M, Linv, diag, m, mp, nb, counters, counters + 1, flags,
-                          reinterpret_cast<unsigned*>(counters + 3), 1e-13};
+                          reinterpret_cast<unsigned*>(counters + 3), chain, 1e-13};
     dense_cholesky<double>(s, st, nullptr);
-    unsigned epoch = 0;
     for (int r = 0; r < nrhs; ++r) {
       double* col = rhs + static_cast<size_t>(r) * m;
       k_copy_pad<<<ceil_div(mp, 128), 128, 0, st>>>(col, z, m, mp);
-      dense_solve<double>(s, z, epoch, counters + 2, st, nullptr);
+      dense_solve<double>(s, z, counters + 2, st, nullptr);
       k_copy_back<<<ceil_div(m, 128), 128, 0, st>>>(z, col, m);
     }
     int h[3] = {0, 0, 0};

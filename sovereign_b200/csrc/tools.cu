@@ -157,17 +157,18 @@ int normal_factor_solve_device(int m, int n, const int* col_ptr, const int* row_
     SOV_CUDA(cudaMemset(err.p, 0, sizeof(int)));
     Tmp<double> z(mp);
     SOV_CUDA(cudaMemset(z.p, 0, sizeof(double) * mp));
-    unsigned epoch = 0;
+    Tmp<double> chain(2 * static_cast<size_t>(mp));
+    dense_chain_reset(chain.p, mp, 0);
     if (precision == SOV_PRECISION_FP64) {
       Tmp<double> M(static_cast<size_t>(mp) * mp), Linv(static_cast<size_t>(nb) * kNB * kNB);
       launch_dense_clear<double>(M.p, m, mp, 0);
       launch_assemble<double>(ad, dx.p, ds.p, nullptr, nullptr, kWeightLp, 1e-12, M.p, ddiag.p, m, mp, 0);
       DenseSystem<double> s{M.p, Linv.p, ddiag.p, m, mp, nb, counters.p, counters.p + 1, flags.p,
-                                reinterpret_cast<unsigned*>(counters.p + 2), 1e-13};
+                                reinterpret_cast<unsigned*>(counters.p + 2), chain.p, 1e-13};
       dense_cholesky<double>(s, 0, nullptr);
       for (int r = 0; r < nrhs; ++r) {
         z.put(rhs + static_cast<size_t>(r) * m, m);
-        dense_solve<double>(s, z.p, epoch, err.p, 0, nullptr);
+        dense_solve<double>(s, z.p, err.p, 0, nullptr);
         z.get(rhs + static_cast<size_t>(r) * m, m);
       }
     } else {
@@ -175,11 +176,11 @@ int normal_factor_solve_device(int m, int n, const int* col_ptr, const int* row_
       launch_dense_clear<float>(M.p, m, mp, 0);
       launch_assemble<float>(ad, dx.p, ds.p, nullptr, nullptr, kWeightLp, 1e-12, M.p, ddiag.p, m, mp, 0);
       DenseSystem<float> s{M.p, Linv.p, ddiag.p, m, mp, nb, counters.p, counters.p + 1, flags.p,
-                               reinterpret_cast<unsigned*>(counters.p + 2), 1e-6};
+                               reinterpret_cast<unsigned*>(counters.p + 2), chain.p, 1e-6};
       dense_cholesky_tc(s, err.p, 0, nullptr);
       for (int r = 0; r < nrhs; ++r) {
         z.put(rhs + static_cast<size_t>(r) * m, m);
-        dense_solve<float>(s, z.p, epoch, err.p, 0, nullptr);
+        dense_solve<float>(s, z.p, err.p, 0, nullptr);
         z.get(rhs + static_cast<size_t>(r) * m, m);
       }
     }
