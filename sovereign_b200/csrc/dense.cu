@@ -48,6 +48,17 @@ __device__ __forceinline__ void load4(const float* p, float v[4]) {
   v[2] = a.z;
   v[3] = a.w;
 }
+// two consecutive elements, aligned to their size together, widened to double
+__device__ __forceinline__ void load2(const double* p, double (&v)[2]) {
+  const double2 a = *reinterpret_cast<const double2*>(p);
+  v[0] = a.x;
+  v[1] = a.y;
+}
+__device__ __forceinline__ void load2(const float* p, double (&v)[2]) {
+  const float2 a = *reinterpret_cast<const float2*>(p);
+  v[0] = a.x;
+  v[1] = a.y;
+}
 // sixteen consecutive elements from 16-byte-aligned global memory, widened to double
 __device__ __forceinline__ void load16(const double* p, double v[16]) {
 #pragma unroll
@@ -677,7 +688,7 @@ void dense_cholesky(const DenseSystem<T>& s, cudaStream_t st, int* launches) {
 // no arithmetic produces; a result with those bits is published as the standard NaN) until then, and a
 // consumer polls the value it needs. Flags cost a chain step two more trips to L2 (fence and flag on
 // one side, flag and then value on the other): FP32 factor of order 700, forward 27.2 -> 19.5 us, backward
-// 25.8 -> 22.9; FP64 of order 2000, forward 71 -> 56 us.
+// 25.8 -> 18.3; FP64 of order 2000, forward 71 -> 56 us, backward 79 -> 53 (its tiles read by columns).
 constexpr int kSolveBatch = 8;  // blocks a triangular-solve block takes per barrier while they lie well behind
 constexpr int kSolveNear = 3;   // the nearest ones are taken one by one, their L loaded before the wait
 constexpr unsigned long long kUnset = ~0ull;  // cudaMemset 0xFF
@@ -773,10 +784,12 @@ __global__ void __launch_bounds__(256) k_trsv_bwd(const T* __restrict__ M, int l
   __shared__ double part[4][kNB];
   __shared__ double xs[kSolveBatch][kNB];
   __shared__ double rhs[kNB];
-  // thread (c, g): column c of the row block's L entries, rows 16g .. 16g+15 of each tile, so a
-  // thread's entries of a tile are 16 consecutive values (vector loads) and the four groups' partial
-  // sums meet in shared memory once per block
-  const int t = threadIdx.x, c = t & (kNB - 1), g = t >> 6;
+  // The last dependency's tile and Linv: thread (c, g) holds column c, rows 16g .. 16g+15, loaded before
+  // any wait. The tiles before it are read along their columns: warp w takes columns 8w .. 8w+7, lanes
+  // two rows each (512 bytes a load; a column per thread touched 32 lines a load), and the lanes'
+  // partial sums meet while the last dependency is still under way.
+  __shared__ double far[kNB];
+  const int t = threadIdx.x, c = t & (kNB - 1), g = t >> 6, lane = t & 31, warp = t >> 5;
   for (int q = blockIdx.x; q < nb; q += gridDim.x) {
     const int i = nb - 1 - q;
     // this thread's entries of Linv_ii and of L_{i+1,i} (the last dependency), loaded before any wait
@@ -790,25 +803,42 @@ __global__ void __launch_bounds__(256) k_trsv_bwd(const T* __restrict__ M, int l
       yi = Y[i * kNB + t];
       Y[i * kNB + t] = __longlong_as_double(static_cast<long long>(kUnset));
     }
-    double acc = 0.0;
     // blocks nb-1 down to i+2
     const int deps = nb - i - 2;
+    double fa[8] = {};
+    const T* tile = M + static_cast<int64_t>(i * kNB + warp * 8) * ld + lane * 2;
     for (int done = 0; done < deps;) {
       const int j0 = nb - 1 - done;
       const int run = solve_run(deps - done);
-      double l[16];
-      load16(colc + j0 * kNB, l);
+      double l[8][2];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) load2(tile + static_cast<int64_t>(e) * ld + j0 * kNB, l[e]);
       for (int idx = t; idx < run * kNB; idx += blockDim.x)
         xs[idx / kNB][idx % kNB] = wait_value(X + (j0 - idx / kNB) * kNB + idx % kNB, err);
       __syncthreads();
-      // acc_c += sum_r L[j*64 + r][i*64 + c] * x_j[r], this thread's 16 rows r
       for (int b = 0; b < run; ++b) {
+        const double x0 = xs[b][lane * 2], x1 = xs[b][lane * 2 + 1];
 #pragma unroll
-        for (int u = 0; u < 16; ++u) acc += l[u] * xs[b][g * 16 + u];
-        if (b + 1 < run) load16(colc + (j0 - b - 1) * kNB, l);
+        for (int e = 0; e < 8; ++e) {
+          fa[e] += l[e][0] * x0;
+          fa[e] += l[e][1] * x1;
+        }
+        if (b + 1 < run)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) load2(tile + static_cast<int64_t>(e) * ld + (j0 - b - 1) * kNB, l[e]);
       }
       __syncthreads();
       done += run;
+    }
+    double acc = 0.0;
+    if (deps > 0) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const double v = warp_sum(fa[e]);
+        if (lane == 0) far[warp * 8 + e] = v;
+      }
+      __syncthreads();
+      if (g == 0) acc = far[c];
     }
     if (i + 1 < nb) {
       if (t < kNB) xs[0][t] = wait_value(X + (i + 1) * kNB + t, err);
@@ -874,7 +904,7 @@ void dense_solve(const DenseSystem<T>& s, double* z, int* err, cudaStream_t st, 
 // the rows of A used to go through a forward and a backward launch each, 33 us a row (portfolio QP of
 // 25 rows, order 448: 16.8 -> 7.3 ms per solve of 12 iterations).
 // ---------------------------------------------------------------------------------------------
-constexpr int kRhsTile = 32;
+constexpr int kRhsTile = 8;  // 8 rather than 32 columns: a chain step's arithmetic shrinks with it (104 -> 59 us)
 
 __global__ void __launch_bounds__(256) k_trsm_fwd(const double* __restrict__ M, int ld, const double* __restrict__ Linv,
                                                   int nb, double* Y, int ldy, int nrhs, unsigned* flags, int* err) {
