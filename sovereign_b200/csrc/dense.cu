@@ -371,6 +371,9 @@ __device__ void potrf_core(T* __restrict__ M, int ld, int kb, const double* __re
     while ((ti + 1) * (ti + 2) / 2 <= u) ++ti;
     tj = u - ti * (ti + 1) / 2;
   }
+  int dq = 0;  // tid < 36: entry (dq, dc) of an 8 x 8 lower triangle
+  while (tid < kPanel * (kPanel + 1) / 2 && (dq + 1) * (dq + 2) / 2 <= tid) ++dq;
+  const int dc = tid - dq * (dq + 1) / 2;
   if (tid < kNB) factor_panel<false, T>(A, Lt0, rinv, dref, 0, r0, m, drop_tol, drops, bad);
   __syncthreads();
   for (int p = 0; p + 1 < kNB / kPanel; ++p) {
@@ -380,13 +383,10 @@ __device__ void potrf_core(T* __restrict__ M, int ld, int kb, const double* __re
     if (tid < kNB) {
       // panel p's update of panel p+1's diagonal block, one entry per thread, shared through A
       if (tid < kPanel * (kPanel + 1) / 2) {
-        int q = 0;
-        while ((q + 1) * (q + 2) / 2 <= tid) ++q;
-        const int c = tid - q * (q + 1) / 2;
-        T a = A[K0 + q][K0 + c];
+        T a = A[K0 + dq][K0 + dc];
 #pragma unroll
-        for (int k = 0; k < kPanel; ++k) a -= Lc[k][K0 + q] * Lc[k][K0 + c];
-        A[K0 + q][K0 + c] = a;
+        for (int k = 0; k < kPanel; ++k) a -= Lc[k][K0 + dq] * Lc[k][K0 + dc];
+        A[K0 + dq][K0 + dc] = a;
       }
       asm volatile("bar.sync 1, 64;" ::: "memory");  // warps 0-1: the diagonal block is updated
       factor_panel<true, T>(A, Ln, rinv, dref, K0, r0, m, drop_tol, drops, bad);
@@ -480,11 +480,15 @@ __global__ void __launch_bounds__(256) k_potrf_diag(T* __restrict__ M, int ld, i
   potrf_block<T>(M, ld, kb, diag, m, Linv, drop_count, fail, drop_tol, potrf_raw);
 }
 
+// Rows of the slices in shared memory: 68 doubles apart, so that an MMA fragment's 8 x 4 entries (four
+// rows, eight entries each) meet in no bank more than twice.
+constexpr int kSliceLd = 68;
+
 // acc[p][q] += sum_k Xs[k][tx + 16 p] Ys[k][ty + 16 q], tx = tid % 16, ty = tid / 16 (256 threads):
 // a half-warp reads 16 consecutive entries of Xs (one wavefront) and one entry of Ys (broadcast),
 // and its results are 16 consecutive rows of a column-major tile (coalesced stores)
 template <class T>
-__device__ __forceinline__ void tile_nt(const T (*Xs)[kNB], const T (*Ys)[kNB], T (&acc)[4][4]) {
+__device__ __forceinline__ void tile_nt(const T (*Xs)[kSliceLd], const T (*Ys)[kSliceLd], T (&acc)[4][4]) {
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll 8
   for (int k = 0; k < kNB; ++k) {
@@ -504,7 +508,7 @@ __device__ __forceinline__ void tile_nt(const T (*Xs)[kNB], const T (*Ys)[kNB], 
 // Two 64 x 64 slices into shared memory, dst[k][r] = src[k * ld + r], on 256 threads with 16
 // loads in flight per thread; kBypassL1 reads past L1 (data written by other CTAs of this launch).
 template <bool kBypassL1, class T>
-__device__ __forceinline__ void load_slices(T (*Xs)[kNB], const T* __restrict__ xsrc, int64_t xld, T (*Ys)[kNB],
+__device__ __forceinline__ void load_slices(T (*Xs)[kSliceLd], const T* __restrict__ xsrc, int64_t xld, T (*Ys)[kSliceLd],
                                             const T* __restrict__ ysrc, int64_t yld) {
   const int tid = threadIdx.x;
 #pragma unroll
@@ -522,6 +526,37 @@ __device__ __forceinline__ void load_slices(T (*Xs)[kNB], const T* __restrict__ 
       Xs[idx / kNB][idx % kNB] = vx[u];
       Ys[idx / kNB][idx % kNB] = vy[u];
     }
+  }
+}
+
+// Products of 64 x 64 slices where a triangle of them is zero or not wanted, in 8 x 8 FP64 MMA tiles: 36 of
+// the 64 tiles' work, which is what bounds them (one SM: 4096 cycles for the whole product). Warp w has
+// row block rb; its lane (q, t) = (lane / 4, lane % 4) holds entries (8 rb + q, 8 cb + 2t) and the next one
+// of column block cb in c[cb].
+__device__ __forceinline__ void mma_step(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
+// c += X Y' with Y lower triangular: Xs[k][r], Ys[k][col] = 0 for k > col
+__device__ __forceinline__ void product_lower_factor(const double (*Xs)[kSliceLd], const double (*Ys)[kSliceLd], int rb,
+                                                     double (&c)[8][2]) {
+  const int q = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+  double a[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) a[k] = Xs[4 * k + t][8 * rb + q];
+#pragma unroll
+  for (int k = 0; k < 16; ++k)
+#pragma unroll
+    for (int cb = k / 2; cb < 8; ++cb) mma_step(c[cb], a[k], Ys[4 * k + t][8 * cb + q]);
+}
+// the column blocks cb <= rb of c += X X'
+__device__ __forceinline__ void product_lower_result(const double (*Xs)[kSliceLd], int rb, double (&c)[8][2]) {
+  const int q = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+#pragma unroll 4
+  for (int k = 0; k < 16; ++k) {
+    const double a = Xs[4 * k + t][8 * rb + q];
+#pragma unroll
+    for (int cb = 0; cb < 8; ++cb)
+      if (cb <= rb) mma_step(c[cb], a, Xs[4 * k + t][8 * cb + q]);
   }
 }
 
@@ -556,14 +591,18 @@ __device__ __forceinline__ void tile_triangle(int t, int& ii, int& jj) {
 // A trailing tile only waits for panel solves, which never wait and hold lower tickets, so every
 // item it waits for was taken by a CTA that is already running. Blocks solved by other CTAs of
 // the launch are read past L1 (ld.global.cg).
-template <class T>
-__global__ void __launch_bounds__(256) k_panel_update(T* __restrict__ M, int ld, int kb, int nb,
-                                                      const double* __restrict__ diag, int m, T* __restrict__ Linv,
+// Item 0 bounds a launch (the other items finish under it): 43000 cycles at 64 x 64, of which the factor and
+// inverse 25000. Its two products take 36 of 64 tiles, the diagonal tile is on its way from the start,
+// and the solved block is released only once the factor can begin (its readers have that long).
+// Measured per panel at order 2000: 28.6 us before, 24.3 in this form (sums in the same order, same bits).
+__global__ void __launch_bounds__(256) k_panel_update(double* __restrict__ M, int ld, int kb, int nb,
+                                                      const double* __restrict__ diag, int m, double* __restrict__ Linv,
                                                       int* drop_count, int* fail, double drop_tol, unsigned* flags,
                                                       unsigned stamp, unsigned* tickets, unsigned base) {
+  using T = double;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T(*Xs)[kNB] = reinterpret_cast<T(*)[kNB]>(smem_raw);
-  T(*Ys)[kNB] = reinterpret_cast<T(*)[kNB]>(smem_raw + sizeof(T) * kNB * kNB);
+  T(*Xs)[kSliceLd] = reinterpret_cast<T(*)[kSliceLd]>(smem_raw);
+  T(*Ys)[kSliceLd] = reinterpret_cast<T(*)[kSliceLd]>(smem_raw + sizeof(T) * kNB * kSliceLd);
   __shared__ unsigned item_s;
   __shared__ int ok_s;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -573,48 +612,57 @@ __global__ void __launch_bounds__(256) k_panel_update(T* __restrict__ M, int ld,
   const int R = nb - kb - 1, k0 = kb * kNB;
   if (item < R) {
     const int i = kb + 1 + item, r0 = i * kNB;
+    const int warp = tid >> 5, q = (tid & 31) >> 2, t = tid & 3;
+    // row blocks so dealt that the two warps of a scheduler share 9 tiles of a lower triangle
+    const int rb = warp < 4 ? warp : 11 - warp;
+    double cur[8][2];  // item 0: the diagonal tile's lower triangle
+#pragma unroll
+    for (int cb = 0; cb < 8; ++cb)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = 8 * rb + q, c = 8 * cb + 2 * t + e;
+        cur[cb][e] = item == 0 && r >= c ? M[static_cast<int64_t>(r0 + c) * ld + r0 + r] : T(0);
+      }
     // Ys[k][c] = Linv[c][k] = Lk[k * 64 + c]
     load_slices<false>(Xs, M + static_cast<int64_t>(k0) * ld + r0, ld, Ys, Linv + static_cast<int64_t>(kb) * kNB * kNB,
                        kNB);
     __syncthreads();
-    T acc[4][4] = {};
-    tile_nt<T>(Xs, Ys, acc);
+    double acc[8][2] = {};
+    product_lower_factor(Xs, Ys, rb, acc);
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
+    for (int cb = 0; cb < 8; ++cb)
 #pragma unroll
-      for (int p = 0; p < 4; ++p) M[static_cast<int64_t>(k0 + ty + 16 * q) * ld + r0 + tx + 16 * p] = acc[p][q];
+      for (int e = 0; e < 2; ++e) M[static_cast<int64_t>(k0 + 8 * cb + 2 * t + e) * ld + r0 + 8 * rb + q] = acc[cb][e];
     __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      st_release(flags + i, stamp);
+    if (item != 0) {
+      if (tid == 0) {
+        __threadfence();
+        st_release(flags + i, stamp);
+      }
+      return;
     }
-    if (item != 0) return;
     // look-ahead: A_ii - L_ik L_ik^T from the block just solved, straight into the diagonal
     // factor's shared-memory tile, then its factor and inverse
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
+    for (int cb = 0; cb < 8; ++cb)
 #pragma unroll
-      for (int p = 0; p < 4; ++p) Xs[ty + 16 * q][tx + 16 * p] = acc[p][q];
-    T cur[4][4];  // the diagonal tile's lower triangle, loaded while the product runs
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        const int r = tx + 16 * p, c = ty + 16 * q;
-        cur[p][q] = r >= c ? M[static_cast<int64_t>(r0 + c) * ld + r0 + r] : T(0);
-      }
+      for (int e = 0; e < 2; ++e) Xs[8 * cb + 2 * t + e][8 * rb + q] = acc[cb][e];
     __syncthreads();
-    T upd[4][4] = {};
-    tile_nt<T>(Xs, Xs, upd);
+    double upd[8][2] = {};
+    product_lower_result(Xs, rb, upd);
     __syncthreads();  // Xs, which the factor's tile overlays, is fully read
     T(*A)[kNB + 1] = reinterpret_cast<T(*)[kNB + 1]>(smem_raw);
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
+    for (int cb = 0; cb < 8; ++cb)
 #pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        const int r = tx + 16 * p, c = ty + 16 * q;
-        A[r][c] = r >= c ? cur[p][q] - upd[p][q] : T(0);
+      for (int e = 0; e < 2; ++e) {
+        const int r = 8 * rb + q, c = 8 * cb + 2 * t + e;
+        A[r][c] = r >= c ? cur[cb][e] - upd[cb][e] : T(0);
       }
+    if (tid == 255) {  // every thread's rows were stored before the last barriers
+      __threadfence();
+      st_release(flags + i, stamp);
+    }
     potrf_core<T>(M, ld, kb + 1, diag, m, Linv, drop_count, fail, drop_tol, smem_raw);
     return;
   }
@@ -655,10 +703,12 @@ std::atomic<unsigned> g_factor_generation{0};
 
 template <class T>
 void dense_cholesky(const DenseSystem<T>& s, cudaStream_t st, int* launches) {
+  static_assert(sizeof(T) == sizeof(double), "FP32 factors go through dense_cholesky_tc");
+  static_assert(2 * kNB * kSliceLd * sizeof(T) <= potrf_smem_bytes<T>(), "slices larger than the factor's shared memory");
   const size_t smem_potrf = potrf_smem_bytes<T>();
-  once_per_device((const void*)k_panel_update<T>, [&] {
+  once_per_device((const void*)k_panel_update, [&] {
     SOV_CUDA(cudaFuncSetAttribute(k_potrf_diag<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_potrf));
-    SOV_CUDA(cudaFuncSetAttribute(k_panel_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_potrf));
+    SOV_CUDA(cudaFuncSetAttribute(k_panel_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_potrf));
   });
   if (s.nb >= (1 << kStampPanelBits)) throw std::runtime_error("dense factor: too many row blocks");
   const unsigned gen = (g_factor_generation.fetch_add(1) & ((1u << (31 - kStampPanelBits)) - 1)) << kStampPanelBits;
@@ -672,7 +722,7 @@ void dense_cholesky(const DenseSystem<T>& s, cudaStream_t st, int* launches) {
     const int R = s.nb - kb - 1;
     const int items = R + R * (R + 1) / 2 - 1;
     const unsigned stamp = 0x80000000u | gen | static_cast<unsigned>(kb);
-    k_panel_update<T><<<items, 256, smem_potrf, st>>>(s.M, s.mp, kb, s.nb, s.diag, s.m, s.Linv, s.drop_count, s.fail,
+    k_panel_update<<<items, 256, smem_potrf, st>>>(s.M, s.mp, kb, s.nb, s.diag, s.m, s.Linv, s.drop_count, s.fail,
                                                        s.drop_tol, s.flags, stamp, s.tickets, base);
     base += static_cast<unsigned>(items);
     ++n;
@@ -1005,7 +1055,6 @@ template void launch_dense_clear<float>(float*, int, int, cudaStream_t);
 template void dense_potrf_block<double>(const DenseSystem<double>&, int, cudaStream_t);
 template void dense_potrf_block<float>(const DenseSystem<float>&, int, cudaStream_t);
 template void dense_cholesky<double>(const DenseSystem<double>&, cudaStream_t, int*);
-template void dense_cholesky<float>(const DenseSystem<float>&, cudaStream_t, int*);
 template void dense_solve<double>(const DenseSystem<double>&, double*, int*, cudaStream_t, int*);
 template void dense_solve<float>(const DenseSystem<float>&, double*, int*, cudaStream_t, int*);
 
