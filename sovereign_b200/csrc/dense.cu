@@ -737,10 +737,13 @@ void dense_cholesky(const DenseSystem<T>& s, cudaStream_t st, int* launches) {
 // A solved block is handed over by its values alone: the buffer they are published in holds kUnset (a NaN
 // no arithmetic produces; a result with those bits is published as the standard NaN) until then, and a
 // consumer polls the value it needs. Flags cost a chain step two more trips to L2 (fence and flag on
-// one side, flag and then value on the other): FP32 factor of order 700, forward 27.2 -> 19.5 us, backward
-// 25.8 -> 18.3; FP64 of order 2000, forward 71 -> 56 us, backward 79 -> 53 (its tiles read by columns).
-constexpr int kSolveBatch = 8;  // blocks a triangular-solve block takes per barrier while they lie well behind
-constexpr int kSolveNear = 3;   // the nearest ones are taken one by one, their L loaded before the wait
+// one side, flag and then value on the other). A block takes its dependencies one by one, the next tile on
+// its way while it waits: taken up to eight to a barrier, the block that publishes next was still busy
+// with its run when its last value came. Forward / backward, us a solve:
+//                         flags        values, runs of 8    values, one by one
+//   FP64, order 2000      71 / 79      56 / 63              31.5 / 39
+//   FP32, order 700       27.2 / 25.8  20 / 20              14.3 / 15.7
+// Above 148 blocks a CTA takes several rows; 148 rather than 296 CTAs (one per SM, for the registers).
 constexpr unsigned long long kUnset = ~0ull;  // cudaMemset 0xFF
 
 __device__ __forceinline__ void publish_value(double* p, double v) {
@@ -761,15 +764,12 @@ __device__ __forceinline__ double wait_value(const double* p, int* err) {
   return __longlong_as_double(static_cast<long long>(u));
 }
 
-// blocks taken at the next barrier when `left` remain before the last one
-__device__ __forceinline__ int solve_run(int left) { return left > kSolveNear ? min(kSolveBatch, left - kSolveNear) : 1; }
-
 // Forward: L y = r, row block order. z holds r; y goes to Y. X (of the last backward solve) is unset again.
 template <class T>
-__global__ void __launch_bounds__(256) k_trsv_fwd(const T* __restrict__ M, int ld, const T* __restrict__ Linv, int nb,
+__global__ void __launch_bounds__(256, 1) k_trsv_fwd(const T* __restrict__ M, int ld, const T* __restrict__ Linv, int nb,
                                                   const double* z, double* Y, double* X, int* err) {
   __shared__ double part[4][kNB];
-  __shared__ double ys[kSolveBatch][kNB];
+  __shared__ double ys[2][kNB];  // by turns: a block's values are read while the next one's are awaited
   __shared__ double rhs[kNB];
   const int t = threadIdx.x, r = t & (kNB - 1), g = t >> 6;
   for (int i = blockIdx.x; i < nb; i += gridDim.x) {
@@ -787,31 +787,31 @@ __global__ void __launch_bounds__(256) k_trsv_fwd(const T* __restrict__ M, int l
     const double zi = t < kNB ? z[i * kNB + t] : 0.0;
     if (t < kNB) X[i * kNB + t] = __longlong_as_double(static_cast<long long>(kUnset));
     double acc = 0.0;
-    for (int done = 0; done < i - 1;) {  // blocks 0 .. i-2
-      const int run = solve_run(i - 1 - done);
-      const T* Lij = M + static_cast<int64_t>(done * kNB) * ld + i * kNB + r;
+    const T* Lij = M + static_cast<int64_t>(g * 16) * ld + i * kNB + r;
+    double next[16];
+    if (i > 1) {
+#pragma unroll
+      for (int u = 0; u < 16; ++u) next[u] = static_cast<double>(Lij[static_cast<int64_t>(u) * ld]);
+    }
+    for (int j = 0; j + 1 < i; ++j) {  // blocks 0 .. i-2
       double l[16];
 #pragma unroll
-      for (int u = 0; u < 16; ++u) l[u] = static_cast<double>(Lij[static_cast<int64_t>(g * 16 + u) * ld]);
-      for (int idx = t; idx < run * kNB; idx += blockDim.x) ys[idx / kNB][idx % kNB] = wait_value(Y + done * kNB + idx, err);
-      __syncthreads();
-      for (int b = 0; b < run; ++b) {
+      for (int u = 0; u < 16; ++u) l[u] = next[u];
+      if (j + 2 < i) {
 #pragma unroll
-        for (int u = 0; u < 16; ++u) acc += l[u] * ys[b][g * 16 + u];
-        if (b + 1 < run) {
-          Lij += static_cast<int64_t>(kNB) * ld;
-#pragma unroll
-          for (int u = 0; u < 16; ++u) l[u] = static_cast<double>(Lij[static_cast<int64_t>(g * 16 + u) * ld]);
-        }
+        for (int u = 0; u < 16; ++u) next[u] = static_cast<double>(Lij[static_cast<int64_t>((j + 1) * kNB + u) * ld]);
       }
+      if (t < kNB) ys[j & 1][t] = wait_value(Y + j * kNB + t, err);
       __syncthreads();
-      done += run;
+#pragma unroll
+      for (int u = 0; u < 16; ++u) acc += l[u] * ys[j & 1][g * 16 + u];
     }
     if (i > 0) {
-      if (t < kNB) ys[0][t] = wait_value(Y + (i - 1) * kNB + t, err);
+      double(&yl)[kNB] = ys[(i - 1) & 1];
+      if (t < kNB) yl[t] = wait_value(Y + (i - 1) * kNB + t, err);
       __syncthreads();
 #pragma unroll
-      for (int u = 0; u < 16; ++u) acc += lp[u] * ys[0][g * 16 + u];
+      for (int u = 0; u < 16; ++u) acc += lp[u] * yl[g * 16 + u];
     }
     part[g][r] = acc;
     __syncthreads();
@@ -828,83 +828,88 @@ __global__ void __launch_bounds__(256) k_trsv_fwd(const T* __restrict__ M, int l
 }
 
 // Backward: L^T x = y, reverse row block order; x goes to X and z, and Y is unset again.
+// Warp w has columns 8w .. 8w+7 of a block, its lane (c, g) rows 16g .. 16g+15 of one of them. The tiles
+// before the last dependency are read along their columns (a load takes 512 bytes of one; 16 consecutive
+// entries per thread touched 32 lines a load: FP64 of order 2000, 79 -> 53 us) and turned in shared
+// memory by the warp that reads them, so that every sum keeps its order.
+constexpr int kTurnGroup = 18;  // 16 rows and 2 of padding: 16-byte reads of the four groups and two columns
+constexpr int kTurnLd = 4 * kTurnGroup;  // meet in no bank
+__device__ __forceinline__ constexpr int turned(int row) { return row + 2 * (row >> 4); }
+
+__device__ __forceinline__ void turn_tile(double (*W)[kTurnLd], const double (&l)[8][2], double (&lt)[16]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) *reinterpret_cast<double2*>(&W[e][turned(2 * lane)]) = make_double2(l[e][0], l[e][1]);
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < 16; u += 2) {
+    const double2 v = *reinterpret_cast<const double2*>(&W[lane >> 2][(lane & 3) * kTurnGroup + u]);
+    lt[u] = v.x;
+    lt[u + 1] = v.y;
+  }
+  __syncwarp();
+}
+// acc += l . v over this lane's 16 rows, v in turned() order
+__device__ __forceinline__ double dot_rows(const double (&l)[16], const double* v, double acc) {
+  const double* p = v + (threadIdx.x & 3) * kTurnGroup;
+#pragma unroll
+  for (int u = 0; u < 16; u += 2) {
+    const double2 x = *reinterpret_cast<const double2*>(p + u);
+    acc += l[u] * x.x;
+    acc += l[u + 1] * x.y;
+  }
+  return acc;
+}
+
 template <class T>
-__global__ void __launch_bounds__(256) k_trsv_bwd(const T* __restrict__ M, int ld, const T* __restrict__ Linv, int nb,
+__global__ void __launch_bounds__(256, 1) k_trsv_bwd(const T* __restrict__ M, int ld, const T* __restrict__ Linv, int nb,
                                                   double* z, double* Y, double* X, int* err) {
+  __shared__ __align__(16) double W[8][8][kTurnLd];
+  __shared__ __align__(16) double xs[2][kTurnLd];
+  __shared__ __align__(16) double rhs[kTurnLd];
   __shared__ double part[4][kNB];
-  __shared__ double xs[kSolveBatch][kNB];
-  __shared__ double rhs[kNB];
-  // The last dependency's tile and Linv: thread (c, g) holds column c, rows 16g .. 16g+15, loaded before
-  // any wait. The tiles before it are read along their columns: warp w takes columns 8w .. 8w+7, lanes
-  // two rows each (512 bytes a load; a column per thread touched 32 lines a load), and the lanes'
-  // partial sums meet while the last dependency is still under way.
-  __shared__ double far[kNB];
-  const int t = threadIdx.x, c = t & (kNB - 1), g = t >> 6, lane = t & 31, warp = t >> 5;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, c = warp * 8 + (lane >> 2), g = lane & 3;
   for (int q = blockIdx.x; q < nb; q += gridDim.x) {
     const int i = nb - 1 - q;
     // this thread's entries of Linv_ii and of L_{i+1,i} (the last dependency), loaded before any wait
     double li[16], lp[16];
-    const T* Li = Linv + static_cast<int64_t>(i) * kNB * kNB + c * kNB + g * 16;
-    load16(Li, li);
-    const T* colc = M + static_cast<int64_t>(i * kNB + c) * ld + g * 16;  // column i*64+c of L
-    if (i + 1 < nb) load16(colc + (i + 1) * kNB, lp);
+    load16(Linv + static_cast<int64_t>(i) * kNB * kNB + c * kNB + g * 16, li);  // rows 16g .. of column c of Linv_ii
+    if (i + 1 < nb) load16(M + static_cast<int64_t>(i * kNB + c) * ld + g * 16 + (i + 1) * kNB, lp);
     double yi = 0.0;
     if (t < kNB) {
       yi = Y[i * kNB + t];
       Y[i * kNB + t] = __longlong_as_double(static_cast<long long>(kUnset));
     }
-    // blocks nb-1 down to i+2
-    const int deps = nb - i - 2;
-    double fa[8] = {};
-    const T* tile = M + static_cast<int64_t>(i * kNB + warp * 8) * ld + lane * 2;
-    for (int done = 0; done < deps;) {
-      const int j0 = nb - 1 - done;
-      const int run = solve_run(deps - done);
-      double l[8][2];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) load2(tile + static_cast<int64_t>(e) * ld + j0 * kNB, l[e]);
-      for (int idx = t; idx < run * kNB; idx += blockDim.x)
-        xs[idx / kNB][idx % kNB] = wait_value(X + (j0 - idx / kNB) * kNB + idx % kNB, err);
-      __syncthreads();
-      for (int b = 0; b < run; ++b) {
-        const double x0 = xs[b][lane * 2], x1 = xs[b][lane * 2 + 1];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          fa[e] += l[e][0] * x0;
-          fa[e] += l[e][1] * x1;
-        }
-        if (b + 1 < run)
-#pragma unroll
-          for (int e = 0; e < 8; ++e) load2(tile + static_cast<int64_t>(e) * ld + (j0 - b - 1) * kNB, l[e]);
-      }
-      __syncthreads();
-      done += run;
-    }
     double acc = 0.0;
-    if (deps > 0) {
+    const T* tile = M + static_cast<int64_t>(i * kNB + warp * 8) * ld + lane * 2;
+    double l[8][2];
+    if (nb - 1 > i + 1) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const double v = warp_sum(fa[e]);
-        if (lane == 0) far[warp * 8 + e] = v;
+      for (int e = 0; e < 8; ++e) load2(tile + static_cast<int64_t>(e) * ld + (nb - 1) * kNB, l[e]);
+    }
+    for (int j = nb - 1; j > i + 1; --j) {  // blocks nb-1 down to i+2
+      double lt[16];
+      turn_tile(W[warp], l, lt);
+      if (j - 1 > i + 1) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) load2(tile + static_cast<int64_t>(e) * ld + (j - 1) * kNB, l[e]);
       }
+      if (t < kNB) xs[j & 1][turned(t)] = wait_value(X + j * kNB + t, err);
       __syncthreads();
-      if (g == 0) acc = far[c];
+      acc = dot_rows(lt, xs[j & 1], acc);
     }
     if (i + 1 < nb) {
-      if (t < kNB) xs[0][t] = wait_value(X + (i + 1) * kNB + t, err);
+      double(&xl)[kTurnLd] = xs[(i + 1) & 1];
+      if (t < kNB) xl[turned(t)] = wait_value(X + (i + 1) * kNB + t, err);
       __syncthreads();
-#pragma unroll
-      for (int u = 0; u < 16; ++u) acc += lp[u] * xs[0][g * 16 + u];
+      acc = dot_rows(lp, xl, acc);
     }
     part[g][c] = acc;
     __syncthreads();
-    if (t < kNB) rhs[t] = yi - (part[0][t] + part[1][t] + part[2][t] + part[3][t]);
+    if (t < kNB) rhs[turned(t)] = yi - (part[0][t] + part[1][t] + part[2][t] + part[3][t]);
     __syncthreads();
-    // x_c = sum_r Linv[r][c] rhs[r] = sum_r Li[c * 64 + r] rhs[r]
-    double x = 0.0;
-#pragma unroll
-    for (int u = 0; u < 16; ++u) x += li[u] * rhs[g * 16 + u];
-    part[g][c] = x;
+    // x_c = sum_r Linv[r][c] rhs[r]
+    part[g][c] = dot_rows(li, rhs, 0.0);
     __syncthreads();
     if (t < kNB) {
       const double v = part[0][t] + part[1][t] + part[2][t] + part[3][t];
@@ -922,9 +927,14 @@ int dataflow_grid(int nb) {
   SOV_CUDA(cudaGetDevice(&dev));
   if (dev >= kMaxDevices) throw std::runtime_error("dense solve: device index beyond the supported 64");
   once_per_device((const void*)&max_blocks, [&] {
-    int sms = 0, per_sm = 0;
+    int sms = 0, per_sm = 1 << 30;
     SOV_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    SOV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trsv_fwd<double>, 256, 0));
+    for (const void* k : {(const void*)k_trsv_fwd<double>, (const void*)k_trsv_bwd<double>, (const void*)k_trsv_fwd<float>,
+                          (const void*)k_trsv_bwd<float>}) {
+      int n = 0;
+      SOV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, 256, 0));
+      per_sm = std::min(per_sm, n);
+    }
     max_blocks[dev] = std::max(1, sms * std::max(1, per_sm));
   });
   std::lock_guard<std::mutex> g(once_mutex());  // the write above happened under this lock
