@@ -519,10 +519,14 @@ def run_batched_warm_start(args):
     import concurrent.futures as cf
     from sovereign_b200.ipm import InteriorPointSolver
     solver = InteriorPointSolver()
+
+    def solve(mdl):  # with diagnostics: without them so small an LP takes the batched kernel
+        return solver.solve(mdl, with_diag=True)
+
     with cf.ThreadPoolExecutor(max_workers=PLAIN_WORKERS) as ex:
-        list(ex.map(solver.solve, models[:2 * PLAIN_WORKERS]))
+        list(ex.map(solve, models[:2 * PLAIN_WORKERS]))
         t0 = time.perf_counter()
-        plain_res = list(ex.map(solver.solve, models))
+        plain_res = list(ex.map(solve, models))
         t_plain = time.perf_counter() - t0
     plain_err = max(abs(p.objective_value - c[2]) / max(1.0, abs(c[2])) for p, c in zip(plain_res, cold)
                     if p.status_name == "OPTIMAL" and c[0] == A.OPTIMAL)
@@ -608,9 +612,12 @@ def main():
         import concurrent.futures as cf
         solver = InteriorPointSolver()
         with cf.ThreadPoolExecutor(max_workers=PLAIN_WORKERS) as ex:
-            list(ex.map(solver.solve, models[:2 * PLAIN_WORKERS]))
+            def solve(mdl):  # with diagnostics: without them so small an LP takes the batched kernel
+                return solver.solve(mdl, with_diag=True)
+
+            list(ex.map(solve, models[:2 * PLAIN_WORKERS]))
             t0 = time.perf_counter()
-            single = list(ex.map(solver.solve, models))
+            single = list(ex.map(solve, models))
             t_plain = time.perf_counter() - t0
         plain = dict(value=len(models) / t_plain, unit=UNIT,
                      sample=f"all {len(models)} LPs through sov_lp_solve (FP64 single-problem engine), "
