@@ -964,10 +964,15 @@ void dense_solve(const DenseSystem<T>& s, double* z, int* err, cudaStream_t st, 
 // the rows of A used to go through a forward and a backward launch each, 33 us a row (portfolio QP of
 // 25 rows, order 448: 16.8 -> 7.3 ms per solve of 12 iterations).
 // ---------------------------------------------------------------------------------------------
+// Both tiles of L a chain step needs are in shared memory (or on their way in registers) before its flag
+// is awaited; read from L2 after it they were half of the chain: 62.6 -> 32.3 us a launch.
 constexpr int kRhsTile = 8;  // 8 rather than 32 columns: a chain step's arithmetic shrinks with it (104 -> 59 us)
 
 __global__ void __launch_bounds__(256) k_trsm_fwd(const double* __restrict__ M, int ld, const double* __restrict__ Linv,
                                                   int nb, double* Y, int ldy, int nrhs, unsigned* flags, int* err) {
+  extern __shared__ __align__(16) unsigned char trsm_raw[];
+  double(*Ls)[kNB] = reinterpret_cast<double(*)[kNB]>(trsm_raw);  // [column][row] of L_ij
+  double(*Lis)[kNB] = Ls + kNB;                                   // and of Linv_ii
   __shared__ __align__(16) double ys[kRhsTile][kNB];
   __shared__ unsigned item_s;
   __shared__ int ok_s;
@@ -978,12 +983,27 @@ __global__ void __launch_bounds__(256) k_trsm_fwd(const double* __restrict__ M, 
   const int i = static_cast<int>(item_s) / tiles, tile = static_cast<int>(item_s) % tiles;
   const int c0 = tile * kRhsTile, cols = min(kRhsTile, nrhs - c0);
   constexpr int C = kRhsTile / 4;  // columns per thread
-  double acc[C] = {};
-  for (int j = 0; j < i; ++j) {
-    const double* Lij = M + static_cast<int64_t>(j * kNB) * ld + i * kNB + r;
-    double l[16];  // the first loads of L do not wait for the flag
+  double acc[C] = {}, yi[C], next[16];
 #pragma unroll
-    for (int u = 0; u < 16; ++u) l[u] = Lij[static_cast<int64_t>(u) * ld];
+  for (int c = 0; c < C; ++c) {
+    const int cc = g * C + c;
+    yi[c] = cc < cols ? Y[static_cast<int64_t>(c0 + cc) * ldy + i * kNB + r] : 0.0;
+  }
+  const double* Li = Linv + static_cast<int64_t>(i) * kNB * kNB + r;
+#pragma unroll
+  for (int u = 0; u < 16; ++u) Lis[g + 4 * u][r] = Li[(g + 4 * u) * kNB];
+  const double* Lij = M + static_cast<int64_t>(g) * ld + i * kNB + r;
+  if (i > 0) {
+#pragma unroll
+    for (int u = 0; u < 16; ++u) next[u] = Lij[static_cast<int64_t>(4 * u) * ld];
+  }
+  for (int j = 0; j < i; ++j) {
+#pragma unroll
+    for (int u = 0; u < 16; ++u) Ls[g + 4 * u][r] = next[u];
+    if (j + 1 < i) {
+#pragma unroll
+      for (int u = 0; u < 16; ++u) next[u] = Lij[static_cast<int64_t>((j + 1) * kNB + 4 * u) * ld];
+    }
     if (t == 0) ok_s = wait_flag(flags + tile * nb + j, 1u);
     __syncthreads();
     if (!ok_s && t == 0) atomicExch(err, 1);
@@ -993,23 +1013,15 @@ __global__ void __launch_bounds__(256) k_trsm_fwd(const double* __restrict__ M, 
       ys[c][r] = c < cols ? __ldcg(Y + static_cast<int64_t>(c0 + c) * ldy + j * kNB + r) : 0.0;
     }
     __syncthreads();
+#pragma unroll 16
+    for (int k = 0; k < kNB; k += 2) {
+      const double l0 = Ls[k][r], l1 = Ls[k + 1][r];
 #pragma unroll
-    for (int k0 = 0; k0 < kNB; k0 += 16) {
-      double nx[16];
-      if (k0 + 16 < kNB)
-#pragma unroll
-        for (int u = 0; u < 16; ++u) nx[u] = Lij[static_cast<int64_t>(k0 + 16 + u) * ld];
-#pragma unroll
-      for (int u = 0; u < 16; u += 2)
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-          const double2 y2 = *reinterpret_cast<const double2*>(&ys[g * C + c][k0 + u]);
-          acc[c] += l[u] * y2.x;
-          acc[c] += l[u + 1] * y2.y;
-        }
-      if (k0 + 16 < kNB)
-#pragma unroll
-        for (int u = 0; u < 16; ++u) l[u] = nx[u];
+      for (int c = 0; c < C; ++c) {
+        const double2 y2 = *reinterpret_cast<const double2*>(&ys[g * C + c][k]);
+        acc[c] += l0 * y2.x;
+        acc[c] += l1 * y2.y;
+      }
     }
     __syncthreads();
   }
@@ -1017,14 +1029,13 @@ __global__ void __launch_bounds__(256) k_trsm_fwd(const double* __restrict__ M, 
 #pragma unroll
   for (int c = 0; c < C; ++c) {
     const int cc = g * C + c;
-    ys[cc][r] = (cc < cols ? Y[static_cast<int64_t>(c0 + cc) * ldy + i * kNB + r] : 0.0) - acc[c];
+    ys[cc][r] = yi[c] - acc[c];
     acc[c] = 0.0;
   }
   __syncthreads();
-  const double* Li = Linv + static_cast<int64_t>(i) * kNB * kNB + r;
-#pragma unroll 8
+#pragma unroll 16
   for (int k = 0; k < kNB; k += 2) {
-    const double l0 = Li[k * kNB], l1 = Li[(k + 1) * kNB];
+    const double l0 = Lis[k][r], l1 = Lis[k + 1][r];
 #pragma unroll
     for (int c = 0; c < C; ++c) {
       const double2 y2 = *reinterpret_cast<const double2*>(&ys[g * C + c][k]);
@@ -1050,7 +1061,11 @@ void dense_forward_multi(const DenseSystem<double>& s, double* Y, int ldy, int n
                          cudaStream_t st, int* launches) {
   if (nrhs <= 0) return;
   SOV_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned) * dense_forward_flags(s.nb, nrhs), st));
-  k_trsm_fwd<<<s.nb * ceil_div(nrhs, kRhsTile), 256, 0, st>>>(s.M, s.mp, s.Linv, s.nb, Y, ldy, nrhs, flags, err);
+  constexpr int smem = 2 * kNB * kNB * sizeof(double);
+  once_per_device((const void*)k_trsm_fwd, [&] {
+    SOV_CUDA(cudaFuncSetAttribute(k_trsm_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  });
+  k_trsm_fwd<<<s.nb * ceil_div(nrhs, kRhsTile), 256, smem, st>>>(s.M, s.mp, s.Linv, s.nb, Y, ldy, nrhs, flags, err);
   SOV_LAUNCH_CHECK();
   if (launches) *launches += 1;
 }
