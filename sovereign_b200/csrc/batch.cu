@@ -1224,8 +1224,6 @@ std::mutex g_tune_mu;
 std::map<int, int> g_tuned_threads;  // bucket mmax -> kernel shape code
 std::map<int, int> g_tuned_per_sm;   // bucket mmax -> resident CTAs per SM it launches (absent: all that fit)
 
-int bucket_of(int m) { return std::max(32, ((m + 31) / 32) * 32); }
-
 // Host worker threads, started once and kept for the life of the process (never destroyed: they
 // wait on a condition variable when idle): the batch builds and publishes run several parallel
 // loops per call, and starting threads for each of them cost milliseconds per call. One loop at a
@@ -1662,24 +1660,7 @@ int sm_count() {
   return sms;
 }
 
-// Width of a bucket's CTAs by the LPs of the batch and their mean columns, where no pin and no
-// autotuned choice says otherwise. While every LP has an SM to itself the widest CTA is fastest
-// (its column and row passes scale, the factor's pivot chain does not: 24 transportation LPs 2.16 ms
-// at 128 threads, 1.46 at 256, 1.07 at 512); up to two LPs an SM, 512 threads only for LPs with many
-// columns (300 transportation LPs 1.98 / 1.85 ms at 256 / 512, 200 nodes of 149 columns 0.61 / 1.10);
-// beyond, the choice is between four LPs of 128 threads on an SM and two of 256: long column passes
-// want the wider (4096 transportation LPs, 1225 columns on average: 17.0 / 13.3 ms at 128 / 256;
-// 1000 of 750 columns 2.8 / 2.5 ms), short ones the more resident LPs (3000 LPs of 324 columns 3.2 /
-// 3.8 ms, 1000 nodes 1.5 / 2.2 ms); up to four LPs an SM the line lies lower (400 LPs of 324 columns
-// 0.90 / 0.73 ms, 400 nodes 0.77 / 1.15 ms).
-int width_for(int total, double mean_cols) {
-  const int sms = sm_count();
-  if (total <= sms) return 512;
-  if (total <= 2 * sms) return mean_cols >= 1000.0 ? 512 : 256;
-  return mean_cols >= (total <= 4 * sms ? 250.0 : 600.0) ? 256 : 128;
-}
-
-int threads_for(int mmax, int total, double mean_cols) {
+int threads_for(int mmax, const BatchCall& call) {
   // SOVEREIGN_BATCH_THREADS=128|129|256|257|512 pins every bucket to a shape (tests run each one
   // this way; odd codes are the lean shapes)
   if (const char* e = std::getenv("SOVEREIGN_BATCH_THREADS")) {
@@ -1691,7 +1672,7 @@ int threads_for(int mmax, int total, double mean_cols) {
   std::lock_guard<std::mutex> g(g_tune_mu);
   auto it = g_tuned_threads.find(mmax);
   if (it != g_tuned_threads.end()) return it->second;
-  return width_for(total, mean_cols);
+  return width_for(sm_count(), call, mmax);
 }
 
 void launch_any(const BatchDev& bd, int mmax, int code, int grid, cudaStream_t st) {
@@ -1731,7 +1712,7 @@ size_t align8(size_t v) { return (v + 7) & ~size_t(7); }
 }  // namespace
 
 Batch* batch_create(int count, const sov_model* models, const sov_options* opt_in, int opt_stride,
-                    const DeviceStarts* starts, int first_lp) {
+                    const DeviceStarts* starts, int first_lp, const BatchCall* call) {
   auto model_no = [&](int i) { return std::to_string(first_lp + i); };  // the caller's numbering
   auto B = std::make_unique<Batch>();
   B->count = count;
@@ -1852,6 +1833,12 @@ Batch* batch_create(int count, const sov_model* models, const sov_options* opt_i
   B->total_pub = pv;
   B->pubdata.alloc(static_cast<size_t>(std::max(1LL, pubn)));
   // buckets by m, each ordered largest-first (cost ~ m^3 + nnz); their orders travel with the inputs
+  BatchCall own;
+  if (!call) {
+    for (int i = 0; i < count; ++i)
+      if (kind[i] != kSingle) own.add(shape[i].m0, shape[i].n_struct);
+    call = &own;
+  }
   std::map<int, std::vector<int>> groups;
   for (int i = 0; i < count; ++i)
     if (B->meta[i].m > 0) groups[bucket_of(B->meta[i].m)].push_back(i);
@@ -1869,7 +1856,7 @@ Batch* batch_create(int count, const sov_model* models, const sov_options* opt_i
     auto bk = std::make_unique<Batch::Bucket>();
     bk->mmax = it->first;
     bk->count = static_cast<int>(ids.size());
-    bk->threads = threads_for(bk->mmax, count, static_cast<double>(nv) / count);
+    bk->threads = threads_for(bk->mmax, *call);
     bk->grid = grid_for(bk->mmax, bk->threads, bk->count);
     order_at.push_back(all_orders.size());
     all_orders.insert(all_orders.end(), ids.begin(), ids.end());
@@ -2353,6 +2340,10 @@ int solve_batch(int count, const sov_model* models, const sov_options* opt, int 
       if (k < parts) acc += taper ? parts - k : 1;
     }
   }
+  BatchCall call;
+  // The model's own sizes: a pass over all bounds for the bound rows of every LP would cost 0.1-0.3 ms
+  // before the first launch, so LPs that only their bound rows take past the kernel's limit count too.
+  for (int i = 0; parts > 1 && i < count; ++i) call.add(models[i].m, models[i].n);
   std::vector<std::unique_ptr<Batch>> batches;
   std::vector<cudaStream_t> streams;
   auto part_lo = [&](int k) { return lo_of[k]; };
@@ -2367,7 +2358,7 @@ int solve_batch(int count, const sov_model* models, const sov_options* opt, int 
                                  ? reinterpret_cast<const sov_options*>(reinterpret_cast<const char*>(opt) +
                                                                         static_cast<size_t>(lo) * opt_stride)
                                  : opt;
-      batches.emplace_back(batch_create(hi - lo, models + lo, o, opt_stride, starts, lo));
+      batches.emplace_back(batch_create(hi - lo, models + lo, o, opt_stride, starts, lo, parts > 1 ? &call : nullptr));
       cudaStream_t st = CudaObjectPool::get().stream(false);
       streams.push_back(st);
       batch_launch(batches.back().get(), st, true);

@@ -5,11 +5,10 @@
 
 #include <string>
 
+#include "batch_width.hpp"
 #include "sov_ipm.h"
 
 namespace sov {
-
-constexpr int kBatchMaxRows = 128;  // IPM rows of an LP the batched kernel takes
 
 struct Batch;
 
@@ -24,9 +23,9 @@ struct DeviceStarts {
 int solve_batch(int count, const sov_model* models, const sov_options* opt, int opt_stride, sov_result* results,
                 const DeviceStarts* starts = nullptr);
 // first_lp: the caller's position of models[0] (a part of a larger call), for the device starts
-// and the model numbers in errors
+// and the model numbers in errors; call: the LPs of that call (null: these are all)
 Batch* batch_create(int count, const sov_model* models, const sov_options* opt, int opt_stride = 0,
-                    const DeviceStarts* starts = nullptr, int first_lp = 0);
+                    const DeviceStarts* starts = nullptr, int first_lp = 0, const BatchCall* call = nullptr);
 void batch_solve(Batch* b, cudaStream_t st);
 void batch_results(Batch* b, sov_result* results);
 void batch_stats(const Batch* b, int* launches, double* kernel_ms, double* bytes, double* flops);

@@ -21,3 +21,7 @@ def run_check(tmp_path, name):
 
 def test_streams_and_events_stay_on_their_device(tmp_path):
     run_check(tmp_path, "handle_pool_check")
+
+
+def test_width_rule(tmp_path):
+    run_check(tmp_path, "batch_width_check")

@@ -104,3 +104,22 @@ def test_single_solve_routes_agree_when_stopped_early_or_warm_started(monkeypatc
     bad.lb, bad.ub = np.full(9, 2.0), np.full(9, 1.0)
     auto, general = both_routes(bad, monkeypatch)
     assert auto.status_name == general.status_name and auto.message == general.message
+
+
+@pytest.mark.parametrize("make,count", [(lambda s: P.transport(18, 18, s), 3072), (lambda s: P.transport(18, 18, s), 500),
+                                        (lambda s: P.transport(30, 12 + s % 9, s), 700)])
+def test_parts_give_the_bits_of_one_batch(make, count, monkeypatch):
+    # each normal-matrix entry has one term here, so an LP's bits depend on its CTA width alone, and that on
+    # the call, not on the part an LP is in
+    pool = [make(s) for s in range(40)]
+    models = [pool[k % 40] for k in range(count)]
+    monkeypatch.setenv("SOVEREIGN_BATCH_PARTS", "1")
+    one = solve_batch(models)
+    monkeypatch.setenv("SOVEREIGN_BATCH_PARTS", "7")
+    parts = solve_batch(models)
+    monkeypatch.delenv("SOVEREIGN_BATCH_PARTS")
+    auto = solve_batch(models)
+    for a, b, c in zip(one, parts, auto):
+        assert a.status_name == "OPTIMAL"
+        assert a.objective_value == b.objective_value == c.objective_value
+        assert np.array_equal(a.primal, b.primal) and np.array_equal(a.primal, c.primal)
