@@ -243,8 +243,10 @@ int sov_batch_stats(const sov_batch* batch, int32_t* launches, double* kernel_ms
 int sov_batch_transfer_bytes(const sov_batch* batch, double* h2d_bytes, double* d2h_bytes);
 void sov_batch_destroy(sov_batch* batch);
 
-/* Batched-kernel schedule chosen by the autotuner for a size bucket (threads per CTA, normal
- * matrix precision). tuning_file may be NULL (in-memory only). */
+/* Batched-kernel schedule chosen by the autotuner for a size bucket (threads per CTA, resident CTAs
+ * per SM), kept for the process. A choice applies to batches with as many LPs per SM as the one it was timed
+ * on (up to 1, 2, 3, 4, or more), so tune on a batch of the size to be solved; other batches, and single
+ * solves through sov_lp_solve, go by the built-in rule. The report is JSON; tuning_file (or NULL) receives it. */
 int sov_autotune(int32_t count, const sov_model* models, const sov_options* opt,
                  const char* tuning_file, char* report, int32_t report_len);
 

@@ -1220,9 +1220,7 @@ struct PinnedArena {
 PinnedArena g_arenas[2];
 std::atomic<unsigned> g_arena_turn{0};
 
-std::mutex g_tune_mu;
-std::map<int, int> g_tuned_threads;  // bucket mmax -> kernel shape code
-std::map<int, int> g_tuned_per_sm;   // bucket mmax -> resident CTAs per SM it launches (absent: all that fit)
+TunedWidths g_tuned;
 
 // Host worker threads, started once and kept for the life of the process (never destroyed: they
 // wait on a condition variable when idle): the batch builds and publishes run several parallel
@@ -1376,6 +1374,7 @@ struct Batch {
   std::vector<Pub> pub;
   HBuf<double> pubdata;
   std::vector<int> fallback;  // LPs too large for the batched kernel
+  int call_lps = 0;           // LPs of the call that the batched kernel solves
   // starts handed over on the device (DeviceStarts), kept for the fallback LPs, which take theirs
   // as host warm starts
   bool has_dstarts = false;
@@ -1660,19 +1659,21 @@ int sm_count() {
   return sms;
 }
 
-int threads_for(int mmax, const BatchCall& call) {
+TunedWidths::Choice width_choice(int mmax, const BatchCall& call) {
   // SOVEREIGN_BATCH_THREADS=128|129|256|257|512 pins every bucket to a shape (tests run each one
   // this way; odd codes are the lean shapes)
   if (const char* e = std::getenv("SOVEREIGN_BATCH_THREADS")) {
     const int t = std::atoi(e);
     for (int code : kShapes)
-      if (t == code) return t;
+      if (t == code) return {t, 0};
   }
-  if (const int t = pinned_threads(mmax)) return t;
-  std::lock_guard<std::mutex> g(g_tune_mu);
-  auto it = g_tuned_threads.find(mmax);
-  if (it != g_tuned_threads.end()) return it->second;
-  return width_for(sm_count(), call, mmax);
+  if (const int t = pinned_threads(mmax)) return {t, 0};
+  const int sms = sm_count();
+  if (call.tuned) {
+    const TunedWidths::Choice c = g_tuned.find(mmax, lps_per_sm(sms, call.lps));
+    if (c.threads) return c;
+  }
+  return {width_for(sms, call, mmax), 0};
 }
 
 void launch_any(const BatchDev& bd, int mmax, int code, int grid, cudaStream_t st) {
@@ -1687,14 +1688,7 @@ void launch_any(const BatchDev& bd, int mmax, int code, int grid, cudaStream_t s
 
 // The grid of a bucket launch: every CTA that fits at once, or at most per_sm of them per SM
 // (fewer resident LPs keep a bucket's per-LP vectors inside L2; the autotuner decides).
-int tuned_per_sm(int mmax) {
-  std::lock_guard<std::mutex> g(g_tune_mu);
-  auto it = g_tuned_per_sm.find(mmax);
-  return it != g_tuned_per_sm.end() ? it->second : 0;
-}
-
-int grid_for(int mmax, int code, int count, int per_sm = -1) {
-  if (per_sm < 0) per_sm = tuned_per_sm(mmax);
+int grid_for(int mmax, int code, int count, int per_sm) {
   int cap;
   switch (code) {
     case 128: cap = max_ctas<128, false>(mmax); break;
@@ -1839,6 +1833,7 @@ Batch* batch_create(int count, const sov_model* models, const sov_options* opt_i
       if (kind[i] != kSingle) own.add(shape[i].m0, shape[i].n_struct);
     call = &own;
   }
+  B->call_lps = call->lps;
   std::map<int, std::vector<int>> groups;
   for (int i = 0; i < count; ++i)
     if (B->meta[i].m > 0) groups[bucket_of(B->meta[i].m)].push_back(i);
@@ -1856,8 +1851,9 @@ Batch* batch_create(int count, const sov_model* models, const sov_options* opt_i
     auto bk = std::make_unique<Batch::Bucket>();
     bk->mmax = it->first;
     bk->count = static_cast<int>(ids.size());
-    bk->threads = threads_for(bk->mmax, *call);
-    bk->grid = grid_for(bk->mmax, bk->threads, bk->count);
+    const TunedWidths::Choice choice = width_choice(bk->mmax, *call);
+    bk->threads = choice.threads;
+    bk->grid = grid_for(bk->mmax, bk->threads, bk->count, choice.per_sm);
     order_at.push_back(all_orders.size());
     all_orders.insert(all_orders.end(), ids.begin(), ids.end());
     B->buckets.push_back(std::move(bk));
@@ -2317,7 +2313,7 @@ void parallel_memcpy(void* dst, const void* src, size_t bytes) {
 }
 
 int solve_batch(int count, const sov_model* models, const sov_options* opt, int opt_stride, sov_result* results,
-                const DeviceStarts* starts) {
+                const DeviceStarts* starts, bool tuned) {
   if (count == 0) return SOV_OK;
   // Large batches in parts, pipelined: each part's graph is launched as soon as its inputs are on
   // the device, so the host standard form and the copies of the next part overlap the solves of the
@@ -2343,7 +2339,9 @@ int solve_batch(int count, const sov_model* models, const sov_options* opt, int 
   BatchCall call;
   // The model's own sizes: a pass over all bounds for the bound rows of every LP would cost 0.1-0.3 ms
   // before the first launch, so LPs that only their bound rows take past the kernel's limit count too.
-  for (int i = 0; parts > 1 && i < count; ++i) call.add(models[i].m, models[i].n);
+  call.tuned = tuned;
+  const bool whole = parts > 1 || !tuned;  // else batch_create's own numbers
+  for (int i = 0; whole && i < count; ++i) call.add(models[i].m, models[i].n);
   std::vector<std::unique_ptr<Batch>> batches;
   std::vector<cudaStream_t> streams;
   auto part_lo = [&](int k) { return lo_of[k]; };
@@ -2358,7 +2356,7 @@ int solve_batch(int count, const sov_model* models, const sov_options* opt, int 
                                  ? reinterpret_cast<const sov_options*>(reinterpret_cast<const char*>(opt) +
                                                                         static_cast<size_t>(lo) * opt_stride)
                                  : opt;
-      batches.emplace_back(batch_create(hi - lo, models + lo, o, opt_stride, starts, lo, parts > 1 ? &call : nullptr));
+      batches.emplace_back(batch_create(hi - lo, models + lo, o, opt_stride, starts, lo, whole ? &call : nullptr));
       cudaStream_t st = CudaObjectPool::get().stream(false);
       streams.push_back(st);
       batch_launch(batches.back().get(), st, true);
@@ -2391,7 +2389,7 @@ std::string autotune(int count, const sov_model* models, const sov_options* opt,
   bool any_free = false;
   for (size_t k = 0; k < B->buckets.size(); ++k) {
     auto& bk = B->buckets[k];
-    if (pinned_threads(bk->mmax)) {  // threads_for gave the pinned shape: nothing to time
+    if (pinned_threads(bk->mmax)) {  // width_choice gave the pinned shape: nothing to time
       alone[k] = "\"pinned\": 1";
       alone_t[k] = bk->threads;
       continue;
@@ -2491,12 +2489,9 @@ std::string autotune(int count, const sov_model* models, const sov_options* opt,
   std::ostringstream rep;
   rep << "{";
   {
-    std::lock_guard<std::mutex> g(g_tune_mu);
     for (size_t k = 0; k < B->buckets.size(); ++k) {
       const auto& bk = B->buckets[k];
-      g_tuned_threads[bk->mmax] = bk->threads;
-      if (per_sm_kept[k] > 0) g_tuned_per_sm[bk->mmax] = per_sm_kept[k];
-      else g_tuned_per_sm.erase(bk->mmax);
+      g_tuned.set(bk->mmax, lps_per_sm(sms, B->call_lps), {bk->threads, per_sm_kept[k]});
       rep << (k ? ", " : "") << "\"m<=" << bk->mmax << "\": {" << alone[k] << ", \"alone\": " << alone_t[k]
           << ", \"chosen\": " << bk->threads << ", \"per_sm\": " << per_sm_kept[k] << ", \"count\": " << bk->count
           << ", \"grid\": " << bk->grid << "}";

@@ -20,8 +20,9 @@ struct DeviceStarts {
   cudaEvent_t ready;  // recorded when the starts are written (or null: already written)
 };
 
+// tuned: the autotuner's choices apply (false: width_for alone)
 int solve_batch(int count, const sov_model* models, const sov_options* opt, int opt_stride, sov_result* results,
-                const DeviceStarts* starts = nullptr);
+                const DeviceStarts* starts = nullptr, bool tuned = true);
 // first_lp: the caller's position of models[0] (a part of a larger call), for the device starts
 // and the model numbers in errors; call: the LPs of that call (null: these are all)
 Batch* batch_create(int count, const sov_model* models, const sov_options* opt, int opt_stride = 0,

@@ -3,6 +3,9 @@
 #pragma once
 
 #include <algorithm>
+#include <map>
+#include <mutex>
+#include <utility>
 
 namespace sov {
 
@@ -16,6 +19,7 @@ inline int bucket_of(int m) { return std::max(32, ((m + 31) / 32) * 32); }
 struct BatchCall {
   int lps = 0, max_cols = 0;  // model columns, without slacks
   double cols = 0.0;
+  bool tuned = true;  // autotuned choices apply
   void add(int rows, int columns) {
     if (rows > kBatchMaxRows || columns <= 0) return;  // another path's
     ++lps;
@@ -56,5 +60,31 @@ inline int width_for(int sms, const BatchCall& call, int mmax) {
   }
   return wide ? 256 : 128;
 }
+
+// LPs per SM of a call: 1 .. 4, 5 for more. The lines of width_for lie between these.
+inline int lps_per_sm(int sms, int lps) { return std::min(5, std::max(1, (lps + sms - 1) / sms)); }
+
+// The autotuner's choices. A choice holds for the size bucket and the LPs per SM it was timed at: the width
+// that is fastest for 4096 LPs costs a batch of 24 or a single LP up to twice its time.
+class TunedWidths {
+ public:
+  struct Choice {
+    int threads = 0;  // 0: none
+    int per_sm = 0;   // resident CTAs per SM (0: all that fit)
+  };
+  Choice find(int mmax, int load) {
+    std::lock_guard<std::mutex> g(mu_);
+    const auto it = choices_.find({mmax, load});
+    return it != choices_.end() ? it->second : Choice{};
+  }
+  void set(int mmax, int load, Choice c) {
+    std::lock_guard<std::mutex> g(mu_);
+    choices_[{mmax, load}] = c;
+  }
+
+ private:
+  std::mutex mu_;
+  std::map<std::pair<int, int>, Choice> choices_;
+};
 
 }  // namespace sov

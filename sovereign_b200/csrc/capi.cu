@@ -103,7 +103,8 @@ struct StreamGuard {
 // with 16000 / 64000 entries 5.2 -> 2.5 / 9.6 -> 7.2, of 100 rows with 160000 entries 22 -> 16.
 // Only LPs in which no two rows share two columns (transportation and assignment LPs): the batched
 // kernel sums a normal-matrix entry's terms with shared-memory atomics, in any order, so with several
-// terms two calls could differ in the last bits, which single solves never did.
+// terms two calls could differ in the last bits, which single solves never did. For the same reason no
+// autotuned width reaches this route (it would sum in another order), besides costing up to twice the time.
 // Callers that ask for what the batched kernel does not keep (diagnostics with their histories, the
 // iterate of a given iteration), another precision or a factorization take the general engine.
 constexpr int kOneCtaEntries = 131072;
@@ -145,7 +146,7 @@ int solve_one(const sov_model* model, const sov_options* opt_in, sov_result* res
     if (rc) throw std::runtime_error(g_last_error);
     if (!qp && takes_batched_kernel(*model, opt, *result)) {
       try {
-        return sov::solve_batch(1, model, &opt, 0, result);
+        return sov::solve_batch(1, model, &opt, 0, result, nullptr, false);
       } catch (const sov::CudaError&) {
         throw;
       } catch (const std::exception&) {

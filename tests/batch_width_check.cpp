@@ -55,6 +55,14 @@ int main() {
   BatchCall few = mixed(24, 10, 60);
   for (int i = 0; i < 3000; ++i) few.add(129 + i, 5000), few.add(5, 0);
   EXPECT(few.lps == 24 && few.max_cols == m24.max_cols && few.cols == m24.cols && width(few, 100) == 512);
+  // autotuned choices stay with the LPs per SM they were timed at
+  sov::TunedWidths tuned;
+  tuned.set(128, sov::lps_per_sm(148, 4096), {256, 1});
+  EXPECT(tuned.find(128, sov::lps_per_sm(148, 3072)).threads == 256 && tuned.find(128, sov::lps_per_sm(148, 593)).per_sm == 1);
+  for (int lps : {1, 24, 148, 149, 296, 297, 444, 445, 592}) EXPECT(tuned.find(128, sov::lps_per_sm(148, lps)).threads == 0);
+  EXPECT(tuned.find(96, sov::lps_per_sm(148, 4096)).threads == 0);
+  tuned.set(128, sov::lps_per_sm(148, 24), {512, 0});
+  EXPECT(tuned.find(128, 1).threads == 512 && tuned.find(128, 5).threads == 256 && sov::lps_per_sm(148, 0) == 1);
   std::printf("failures %d\n", failures);
   return failures != 0;
 }

@@ -1,11 +1,13 @@
 """GPU: the batched kernel at orders around the edges of its 8-column blocks and 32-row groups, at
 every CTA width, with dependent rows among them, against the oracle."""
+import concurrent.futures as cf
+
 import numpy as np
 import pytest
 
 import oracle
 from sovereign_b200 import problems as P
-from sovereign_b200.ipm import InteriorPointOptions, InteriorPointSolver, solve_batch
+from sovereign_b200.ipm import InteriorPointOptions, InteriorPointSolver, autotune, solve_batch
 
 pytestmark = pytest.mark.gpu
 
@@ -123,3 +125,25 @@ def test_parts_give_the_bits_of_one_batch(make, count, monkeypatch):
         assert a.status_name == "OPTIMAL"
         assert a.objective_value == b.objective_value == c.objective_value
         assert np.array_equal(a.primal, b.primal) and np.array_equal(a.primal, c.primal)
+
+
+def test_an_autotune_leaves_other_batch_sizes_and_single_solves_alone():
+    one, few = P.transport(50, 50, 1), P.transport_batch(24, seed=3)
+    before = [InteriorPointSolver().solve(one)] + solve_batch(few)
+    autotune(P.transport_batch(700, seed=5))
+    after = [InteriorPointSolver().solve(one)] + solve_batch(few)
+    autotune(few)  # one LP per SM or less: the single solve's own class
+    after.append(InteriorPointSolver().solve(one))
+    for a, b in zip(before + before[:1], after):
+        assert a.objective_value == b.objective_value and np.array_equal(a.primal, b.primal)
+
+
+def test_single_solves_from_several_threads_give_the_bits_of_one():
+    models = [P.transport(12 + k % 5, 9 + k % 7, k) for k in range(48)] + [P.transport(3, 4, k) for k in range(16)]
+    alone = [InteriorPointSolver().solve(mdl) for mdl in models]
+    with cf.ThreadPoolExecutor(max_workers=8) as ex:
+        together = list(ex.map(InteriorPointSolver().solve, models))
+    for a, b in zip(alone, together):
+        assert "batched" in a.message and a.status_name == "OPTIMAL"
+        assert a.objective_value == b.objective_value and a.iterations == b.iterations
+        assert np.array_equal(a.primal, b.primal) and np.array_equal(a.dual_row, b.dual_row)
