@@ -97,23 +97,27 @@ struct StreamGuard {
 
 // A single small LP as a batch of one: the whole iteration in one CTA of 512 threads, where the general
 // engine launches about 16 kernels and reads its scalars back once per iteration (180 us whatever the
-// size). Up to kBatchMaxRows IPM rows. One SM streams the columns, but the general engine's host set-up
-// grows with them too, so one CTA stays ahead over everything measured (general -> one CTA, a call):
-// 5 x 6 transportation LP 1.35 -> 0.28 ms, 50 x 50 3.4 -> 1.35, 64 x 64 3.6 -> 1.9; LPs of 120 rows
-// with 16000 / 64000 entries 5.2 -> 2.5 / 9.6 -> 7.2, of 100 rows with 160000 entries 22 -> 16.
+// size). Up to kBatchMaxRows IPM rows. Calls, general -> one CTA: 5 x 6 transportation LP 1.35 -> 0.28 ms,
+// 50 x 50 3.4 -> 1.35, 64 x 64 3.6 -> 1.9. One SM streams the columns at about 9 ns an entry and iteration, the
+// general engine's row passes get faster with more rows to spread over the GPU, so the line lies at a product of
+// both (LPs that every row pair of 128, 96, 64, 32 rows gives one column, and single entries beyond): 128 rows, 36256
+// entries 6.0 -> 5.3 ms, 46256 6.5 -> 6.2, 126256 15.3 -> 20.4; 96 rows, 49120 7.7 -> 6.9, 69120 10.8 -> 11.3; 64 rows, 84032
+// 14.2 -> 12.7; 32 rows, 125992 28 -> 17.
 // Only LPs in which no two rows share two columns (transportation and assignment LPs): the batched
 // kernel sums a normal-matrix entry's terms with shared-memory atomics, in any order, so with several
 // terms two calls could differ in the last bits, which single solves never did. For the same reason no
 // autotuned width reaches this route (it would sum in another order), besides costing up to twice the time.
 // Callers that ask for what the batched kernel does not keep (diagnostics with their histories, the
 // iterate of a given iteration), another precision or a factorization take the general engine.
-constexpr int kOneCtaEntries = 131072;
+constexpr int kOneCtaEntries = 131072;          // more was not measured
+constexpr long long kOneCtaRowEntries = 5000000;  // rows x entries
 bool takes_batched_kernel(const sov_model& p, const sov_options& opt, const sov_result& r) {
   if (r.diagnostics || opt.ipm_iterate_at != 0 || opt.precision != SOV_PRECISION_FP64 ||
       opt.factorization != SOV_FACTOR_AUTO)
     return false;
   sov::LpShape sh{};
-  if (!sov::plain_lp_shape(p, &sh) || sh.n <= 0 || sh.m <= 0 || sh.m > sov::kBatchMaxRows || sh.nnz > kOneCtaEntries)
+  if (!sov::plain_lp_shape(p, &sh) || sh.n <= 0 || sh.m <= 0 || sh.m > sov::kBatchMaxRows || sh.nnz > kOneCtaEntries ||
+      static_cast<long long>(sh.m) * sh.nnz > kOneCtaRowEntries)
     return false;
   // pairs of rows met in a column (a bound row meets each other row in its own column only)
   bool met[sov::kBatchMaxRows][sov::kBatchMaxRows] = {};

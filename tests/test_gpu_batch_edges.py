@@ -147,3 +147,25 @@ def test_single_solves_from_several_threads_give_the_bits_of_one():
         assert "batched" in a.message and a.status_name == "OPTIMAL"
         assert a.objective_value == b.objective_value and a.iterations == b.iterations
         assert np.array_equal(a.primal, b.primal) and np.array_equal(a.dual_row, b.dual_row)
+
+
+def complete(m, singles, seed):
+    """Every pair of m rows shares one column; `singles` columns of one entry beyond them."""
+    g = np.random.default_rng(seed)
+    i, j = np.tril_indices(m, -1)
+    cols = np.concatenate([np.repeat(np.arange(i.size), 2), np.arange(i.size, i.size + singles)])
+    rows = np.concatenate([np.stack([j, i], 1).ravel(), g.integers(0, m, singles)]).astype(np.int32)
+    vals, n = g.uniform(0.5, 1.5, cols.size), i.size + singles
+    rhs = np.bincount(rows, weights=vals * g.uniform(0.5, 2.0, n)[cols], minlength=m)
+    return P.Model(n=n, m=m, col_ptr=np.concatenate([[0], np.cumsum(np.bincount(cols, minlength=n))]).astype(np.int32),
+                   row_idx=rows, values=vals, obj=g.uniform(0.5, 2.0, n), rhs=rhs, sense=np.full(m, 2, np.int8),
+                   lb=np.zeros(n), ub=np.full(n, P.INF))
+
+
+@pytest.mark.parametrize("m,singles,batched", [(128, 10000, True), (128, 30000, False), (32, 60000, True)])
+def test_single_solve_route_by_rows_and_entries(m, singles, batched, monkeypatch):
+    # either side of the line beyond which one SM streams the columns slower than the whole GPU
+    auto, general = both_routes(complete(m, singles, 3), monkeypatch)
+    assert ("batched" in auto.message) == batched and "batched" not in general.message
+    assert auto.status_name == general.status_name == "OPTIMAL" and auto.iterations == general.iterations
+    assert abs(auto.objective_value - general.objective_value) <= 1e-9 * abs(general.objective_value)
