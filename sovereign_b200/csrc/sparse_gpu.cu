@@ -5,8 +5,10 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <numeric>
 #include <stdexcept>
+#include <string>
 
 #include "common.cuh"
 
@@ -355,17 +357,19 @@ void SparseFactor::upload(const SparseSymbolic& s, int* drop_count, int* fail, d
   SOV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, k_sparse_solve, kSparseThreads, 0));
   // one CTA per SM: most levels hold few columns, and a grid barrier costs more with more CTAs
   grid_ = std::max(1, sms * std::min(1, std::min(per_sm, per_sm2)));
-  // One CTA where the levels' barriers outweigh what one SM streams. Grid form: 4.2 us a barrier,
-  // two barriers a level. One CTA, measured: solve 1.3 us a level and sweep, plus about 2 ns an
-  // entry of L, and its right-hand side has to fit in shared memory; factor 2 us a level plus about
-  // 4 ns an update term. Solve / factor, grid -> one CTA: chain QP of KKT order 16251 (64 levels,
-  // nnz(L) 44059) 564 -> 232 / 539 -> 465 us; order 26001 (70 levels, nnz(L) 70585) 616 -> 463 us /
-  // 590 against 666 us, so its factor stays on the grid; 60 x 60 grid LP (212 levels) 1.9 -> 0.94 ms.
   int smem_max = 0;
   SOV_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const size_t smem = cta_solve_smem(m, levels);
-  cta_factor_ = static_cast<long long>(S.up_col.size()) <= 1600LL * levels;
-  cta_solve_ = smem <= static_cast<size_t>(smem_max) && nnz_l_ <= 3000LL * levels;
+  cta_factor_ = factor_on_one_cta(m, levels, static_cast<long long>(S.up_col.size()));
+  cta_solve_ = smem <= static_cast<size_t>(smem_max) && solve_on_one_cta(m, levels, nnz_l_);
+  // SOVEREIGN_SPARSE_WALK=grid|cta: one form for every matrix it can take (the tests compare the two)
+  if (const char* e = std::getenv("SOVEREIGN_SPARSE_WALK")) {
+    const bool cta = std::string(e) == "cta";
+    if (cta || std::string(e) == "grid") {
+      cta_factor_ = cta;
+      cta_solve_ = cta && smem <= static_cast<size_t>(smem_max);
+    }
+  }
   if (cta_solve_) {
     d_.fval = put(bufs_, std::vector<double>(s.li.size(), 0.0), st);
     SOV_CUDA(cudaStreamSynchronize(st));
