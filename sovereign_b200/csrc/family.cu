@@ -7,6 +7,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <stdexcept>
 #include <string>
@@ -930,6 +931,7 @@ class Family {
   std::vector<StdForm> forms_;
   cudaStream_t st_ = nullptr;
   size_t smem_max_ = 0;
+  bool cta_solve_ = true;  // a CTA per LP
   int sms_ = 148, per_sm_factor_ = 1, per_sm_solve_ = 1;
   // shared structure
   SparseSymbolic sym_;
@@ -1114,6 +1116,12 @@ void Family::setup_shared(const StdForm& f) {
   int smem_max = 0;
   SOV_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   smem_max_ = static_cast<size_t>(smem_max);
+  cta_solve_ = family_solve_on_one_cta(f.m, S.levels + ceil_div(tail_, kSolvePanel));
+  // SOVEREIGN_FAMILY_SOLVE=grid|cta: one form for every order it can take (the tests compare the two)
+  if (const char* e = std::getenv("SOVEREIGN_FAMILY_SOLVE")) {
+    if (std::string(e) == "grid") cta_solve_ = false;
+    if (std::string(e) == "cta") cta_solve_ = true;
+  }
   once_per_device((const void*)k_fam_solve_lp, [&] {
     SOV_CUDA(cudaFuncSetAttribute(k_fam_solve_lp, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
   });
@@ -1235,9 +1243,9 @@ void Family::factor() {
 
 void Family::solve(double* z) {
   FamSparse f = sp_;
-  // a CTA per LP while an LP's two vectors fit in shared memory (order 12000 and more do)
+  // a CTA per LP where it is the faster form and an LP's two vectors fit in shared memory (up to order 14500)
   const size_t smem = 2 * sizeof(double) * static_cast<size_t>(f.m);
-  if (smem <= smem_max_) {
+  if (smem <= smem_max_ && cta_solve_) {
     k_fam_solve_lp<<<f.W, kLpThreads, smem, st_>>>(f, z);
     SOV_LAUNCH_CHECK();
     return;

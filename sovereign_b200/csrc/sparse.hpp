@@ -142,4 +142,11 @@ inline bool solve_on_one_cta(int columns, int levels, long long nnz_l) {
   return nnz_l <= 3000LL * levels && (columns <= 4000 || columns <= (columns <= 14000 ? 2000LL : 1200LL) * levels);
 }
 
+// The family path's solves on one CTA of 512 threads per LP instead of the whole grid over all LPs: the same trade
+// (steps: the schedule's levels and the dense block's panels, each with its barriers). Solve in us, grid / CTA per LP, 2
+// and 64 LPs: multicommodity of 1800 rows (456 in the dense block) 970 / 244 and 1436 / 363; 60 x 60 grid 2227 /
+// 598 and 2522 / 837; blocks of rows: 2000 in 2 levels 15 / 12 and 16 / 15, 6000 in 8 levels 50 / 41 and 52 / 53, 6000 in one
+// level 9 / 13 and 16 / 21, 14000 in 8 levels 53 / 87 and 91 / 158, in 2 levels 16 / 45 and 52 / 102.
+inline bool family_solve_on_one_cta(int columns, int steps) { return columns <= 2000 || columns <= 700LL * steps; }
+
 }  // namespace sov

@@ -33,6 +33,10 @@ int main() {
   EXPECT(factor_on_one_cta(16251, 64, 1600 * 64) && solve_on_one_cta(16251, 64, 44059));
   EXPECT(!factor_on_one_cta(26001, 70, 1600 * 70 + 1) && solve_on_one_cta(26001, 70, 70585));
   EXPECT(!solve_on_one_cta(3600, 10, 30001));
+  // family solves: a CTA per LP but for many rows in few steps
+  using sov::family_solve_on_one_cta;
+  EXPECT(family_solve_on_one_cta(1800, 40) && family_solve_on_one_cta(2000, 2) && family_solve_on_one_cta(3600, 212));
+  EXPECT(!family_solve_on_one_cta(6000, 8) && !family_solve_on_one_cta(6000, 1) && !family_solve_on_one_cta(14000, 8));
   std::printf("failures %d\n", failures);
   return failures != 0;
 }
