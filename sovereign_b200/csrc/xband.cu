@@ -8,8 +8,8 @@
 // pentadiagonal IPM); its generic QP IPM (:2848-3116) stalls on it, and so do FP64 normal equations:
 // near the optimum the row weights z/w span more than 1e25, so Q's contribution to
 // K = Q + A' diag(z/w) A vanishes below FP64 rounding of the large entries, and the multipliers z
-// (up to ~1e7) leave A'z accurate only to ~1e-9. Here K is assembled, factored (banded L D L', one
-// dependent chain of n columns) and solved in double-double, and x, z, the residuals b - Ax + w and
+// (up to ~1e7) leave A'z accurate only to ~1e-9. Here K is assembled, factored (block L D L' in an
+// odd-even order) and solved in double-double, and x, z, the residuals b - Ax + w and
 // Qx + c - A'z, and the direction's dw = A dx + rp and dz are carried in double-double too; the
 // slack w, step lengths, mu and sigma stay FP64.
 //
@@ -22,7 +22,7 @@
 // d_res = |rd|_inf / max(1, |c|_inf + |Qx|_inf), gap = w'z / (1 + |objective|).
 //
 // The whole solve is one launch of one thread-block cluster (16 CTAs where the device can place
-// one): the vector passes are spread over all its threads, scalars are folded through distributed
+// one, 4 up to 1024 columns): the vector passes are spread over all its threads, scalars are folded through distributed
 // shared memory, and K is factored and solved by odd-even block reduction (reduce_level below).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -45,6 +45,8 @@ namespace {
 
 constexpr int kXbThreads = 512;   // per CTA
 constexpr int kXbCluster = 16;    // CTAs of the cluster (8, the portable size, where 16 cannot be placed)
+constexpr int kXbSmallCluster = 4;  // with few columns
+constexpr int kXbSmall = 1024;
 constexpr int kXbMaxLevels = 32;
 constexpr int kXbTop = 320;       // levels of at most this many blocks run in CTA 0 alone
 
@@ -99,14 +101,14 @@ __device__ __forceinline__ void st_dd(double* h, double* l, long long i, dd v) {
 //   x_o = L'^-1 d^-1 (q - X x_{o-1} - U x_{o+1}).
 // This is the block L D L' of K in an odd-even (nested dissection) order, with the blocks factored
 // rather than inverted: as stable as the natural order (d.natural = 1, SOVEREIGN_XBAND_SEGMENTS=1,
-// runs that one on one thread). About 14 levels at n = 20002 replace chains of hundreds of
+// runs that one on one thread; there is no other number of segments to choose). About 14 levels at n = 20002 replace chains of hundreds of
 // dependent double-double steps: what bounds a solve is the latency of one step per level.
 // A level is two steps: one thread per odd block factors it and solves for X and U (factor_odd),
 // then one thread per entry of the next level's blocks and right-hand sides forms it from both
 // neighbours (update_even): the arithmetic of a level, about 1100 FP64 instructions per pair of
 // blocks, is spread over all threads and its dependent chain is a few double-double operations.
 // Levels are separated by cluster barriers until kXbTop blocks are left; the rest runs in CTA 0.
-// Measured on the device (n = 20002, 83 iterations): one CTA with 512 segments and a serial
+// Measured on the device (n = 20002, 81 iterations): one CTA with 512 segments and a serial
 // separator chain 300 ms; one thread per even block doing a whole level 20.3 ms; this form 17.0 ms.
 template <int KD>
 __device__ __forceinline__ void load_sym(const XbDev& d, long long at, dd (&A)[KD][KD]) {
@@ -793,7 +795,9 @@ __global__ void k_xband_start(XbDev d) {
   }
 }
 
-// One cluster of kXbCluster CTAs (an opt-in size), or of 8 where the device cannot place that one.
+// One cluster of kXbCluster CTAs (an opt-in size), or of 8 where the device cannot place that one. Up to kXbSmall
+// columns 4: its barriers and reductions cost less, and the passes gain nothing from more (4 / 16 CTAs: 3 columns
+// 0.138 / 0.179 ms, 20 0.364 / 0.421, 200 1.51 / 1.59, 1000 3.81 / 3.92; 1500 of half-bandwidth 2 1.15 / 1.14).
 template <int KD>
 void launch_ipm(const XbDev& d, cudaStream_t st) {
   static int ctas[kMaxDevices] = {};
@@ -819,7 +823,7 @@ void launch_ipm(const XbDev& d, cudaStream_t st) {
   });
   {
     std::lock_guard<std::mutex> g(once_mutex());  // the write above happened under this lock
-    at.val.clusterDim.x = static_cast<unsigned>(ctas[dev]);
+    at.val.clusterDim.x = static_cast<unsigned>(d.n <= kXbSmall ? kXbSmallCluster : ctas[dev]);
   }
   cfg.gridDim = dim3(at.val.clusterDim.x);
   SOV_CUDA(cudaLaunchKernelEx(&cfg, k_xband_ipm<KD>, d));

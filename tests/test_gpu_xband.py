@@ -52,3 +52,13 @@ def test_odd_even_reduction_matches_natural_order(kd, blocks, extra, monkeypatch
     assert nat.status_name == "OPTIMAL" and nat.iterations == r.iterations
     assert np.linalg.norm(r.primal - nat.primal) <= 1e-11 * np.linalg.norm(nat.primal)
     assert np.linalg.norm(r.dual_row - nat.dual_row) <= 1e-11 * np.linalg.norm(nat.dual_row)
+
+
+@pytest.mark.parametrize("n", [1023, 1024, 1025])
+def test_cluster_sizes_agree_with_natural_order_at_their_line(n, monkeypatch):
+    mdl = band_qp(n, 2, n)[0]
+    r = QpInteriorPointSolver().solve(mdl)
+    monkeypatch.setenv("SOVEREIGN_XBAND_SEGMENTS", "1")
+    nat = QpInteriorPointSolver().solve(mdl)
+    assert r.status_name == nat.status_name == "OPTIMAL" and nat.iterations == r.iterations
+    assert np.linalg.norm(r.primal - nat.primal) <= 1e-11 * np.linalg.norm(nat.primal)
