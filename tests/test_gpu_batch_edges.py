@@ -169,3 +169,18 @@ def test_single_solve_route_by_rows_and_entries(m, singles, batched, monkeypatch
     assert ("batched" in auto.message) == batched and "batched" not in general.message
     assert auto.status_name == general.status_name == "OPTIMAL" and auto.iterations == general.iterations
     assert abs(auto.objective_value - general.objective_value) <= 1e-9 * abs(general.objective_value)
+
+
+def test_batch_matches_the_general_engine():
+    # with diagnostics a single solve takes the general engine, so two codes are compared (a solve without
+    # them would be a batch of one)
+    models = P.transport_batch(8, seed=9) + [P.transport(64, 64, 2), P.random_sparse_lp(40, 90, 3, 4)]
+    for limit in (250, 5):
+        options = InteriorPointOptions(max_iterations=limit)
+        for mdl, b in zip(models, solve_batch(models, options)):
+            s = InteriorPointSolver(options).solve(mdl, with_diag=True)
+            assert "batched" not in s.message and s.diagnostics["history_iterations"][:2] == [1, 2]
+            assert b.status_name == s.status_name and b.iterations == s.iterations
+            # the same iteration, another order of sums; both stop at a relative gap of 1e-9
+            assert abs(b.objective_value - s.objective_value) <= 1e-9 * abs(s.objective_value)
+            assert np.linalg.norm(b.primal - s.primal) <= 1e-6 * np.linalg.norm(s.primal)
