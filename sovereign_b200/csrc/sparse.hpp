@@ -126,17 +126,18 @@ SparsePieces row_pieces(const std::vector<int>& ptr, int* slots);
 
 // One CTA instead of the grid, where the levels' barriers outweigh what one SM streams. The grid form takes
 // about 5 us a level and factor, or a level and solve (two barriers each). One CTA takes 2 us a level and factor, 1.3 us a level
-// and sweep, plus, on one SM, about 4 ns an update term or 2 ns an entry of L, and its pass over the columns of
+// and sweep, plus, on one SM, its share of the update terms or of the entries of L, and its pass over the columns of
 // a level of more than its 1024 threads, which grows with the whole factor as that leaves the SM's caches. Factor / solve in us,
 // grid -> one CTA:
-//  - terms and entries: chain QP of KKT order 16251 (64 levels, nnz(L) 44059) 539 -> 465 / 564 -> 232; order 26001
-//    (70 levels, nnz(L) 70585) 590 -> 666 / 616 -> 463, so its factor stays on the grid; 60 x 60 grid LP (212 levels,
-//    nnz(L) 55898) 1116 -> 1250 / 1834 -> 650;
+//  - terms and entries: chain QPs of KKT order 3901 (50 levels, 29009 terms, nnz(L) 10447) 282 -> 125 / 427 -> 122, 16251 (64,
+//    123845, 44059) 460 -> 330 / 622 -> 205, 26001 (70, 198695, 70585) 557 -> 476 / 630 -> 332, 45501 (76, 347961, 123556; the
+//    right-hand side does not fit) factor 659 -> 678; grid LPs 40 x 40 (157, 268119, 19755) 781 -> 422 / 901 -> 446, 50 x 50 (171,
+//    573704, 36293) 868 -> 745 / 1436 -> 497, 60 x 60 (212, 1019338, 55898) 1188 -> 1220 / 1769 -> 636;
 //  - columns a level (blocks of 1 to 32 rows): 4000 rows in 1, 2, 4 levels 6.5 -> 5.7 / 8.3 -> 7.8, 11.1 -> 8.7 / 14.5 -> 10.5, 19.7 ->
 //    12.2 / 25.4 -> 13.9; 8000 rows in 1, 4, 8 levels 6.5 -> 8.3 / 7.8 -> 11.0, 20.5 -> 21.4 / 26.1 -> 21.4, 40 -> 32 / 52 -> 32; 20000 rows in
 //    8, 16, 32 levels 40 -> 79 / 63 -> 69, 86 -> 138 / 131 -> 127, 173 -> 140 / 262 -> 138; 27000 rows in 16 levels 87 -> 161 / 137 -> 182.
 inline bool factor_on_one_cta(int columns, int levels, long long terms) {
-  return terms <= 1600LL * levels && (columns <= 4000 || columns <= (columns <= 10000 ? 1000LL : 800LL) * levels);
+  return terms <= 3600LL * levels && (columns <= 4000 || columns <= (columns <= 10000 ? 1000LL : 800LL) * levels);
 }
 inline bool solve_on_one_cta(int columns, int levels, long long nnz_l) {
   return nnz_l <= 3000LL * levels && (columns <= 4000 || columns <= (columns <= 14000 ? 2000LL : 1200LL) * levels);

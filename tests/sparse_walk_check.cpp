@@ -21,7 +21,7 @@ int main() {
   auto solve = [](int m, int b) { return solve_on_one_cta(m, b, m - m / b); };
   for (int m : {500, 1000, 2000, 4000})
     for (int b : {4, 8, 16, 32}) EXPECT(factor(m, b) && solve(m, b));
-  EXPECT(factor(4000, 1) && solve(4000, 1) && solve(4000, 2));
+  EXPECT(factor(4000, 1) && solve(4000, 1) && factor(4000, 2) && solve(4000, 2));
   // wide and shallow: the grid
   for (int m : {8000, 14000, 20000, 27000, 200000})
     for (int b : {1, 2}) EXPECT(!factor(m, b) && !solve(m, b));
@@ -30,8 +30,10 @@ int main() {
   EXPECT(factor(8000, 8) && factor(20000, 32) && !factor(27000, 32));
   EXPECT(solve(8000, 8) && solve(14000, 8) && solve(20000, 32) && !solve(20000, 8) && !solve(27000, 16));
   // deep: by terms and entries
-  EXPECT(factor_on_one_cta(16251, 64, 1600 * 64) && solve_on_one_cta(16251, 64, 44059));
-  EXPECT(!factor_on_one_cta(26001, 70, 1600 * 70 + 1) && solve_on_one_cta(26001, 70, 70585));
+  EXPECT(factor_on_one_cta(16251, 64, 123845) && solve_on_one_cta(16251, 64, 44059));
+  EXPECT(factor_on_one_cta(26001, 70, 198695) && solve_on_one_cta(26001, 70, 70585));
+  EXPECT(!factor_on_one_cta(45501, 76, 347961) && !factor_on_one_cta(3600, 212, 1019338));
+  EXPECT(factor_on_one_cta(2500, 171, 573704) && solve_on_one_cta(3600, 212, 55898));
   EXPECT(!solve_on_one_cta(3600, 10, 30001));
   // family solves: a CTA per LP but for many rows in few steps
   using sov::family_solve_on_one_cta;
