@@ -7,7 +7,7 @@
 // m = 128, so up to three LPs share an SM) lives in shared memory and is factored there as L D L'
 // with the reference's dependent-row rule; n-vectors stay in global memory, where
 // the working set of the resident CTAs fits in the 126 MB L2. Size buckets (by m) get their own
-// launch with a shared-memory footprint and thread count chosen per bucket by the autotuner; the
+// launch with a shared-memory footprint and a thread count by width_for or the autotuner; the
 // bucket launches of a batch run concurrently on forked streams, captured once in a CUDA graph.
 #include <unistd.h>
 
@@ -2318,7 +2318,7 @@ int solve_batch(int count, const sov_model* models, const sov_options* opt, int 
   // Large batches in parts, pipelined: each part's graph is launched as soon as its inputs are on
   // the device, so the host standard form and the copies of the next part overlap the solves of the
   // ones before; the results are read back in order once all parts are launched. A part's LPs are
-  // solved exactly as in one batch (per-LP work, bucket widths by m).
+  // solved exactly as in one batch (per-LP work, bucket widths by the whole call).
   // 4096 LPs per call (medians of 5-7 calls, results read back behind the solves, two stagings):
   // 4 parts 18.8-19.9 ms, 6 parts 18.4-19.2, 8 parts 18.2-18.3, 10 parts 19.5
   int parts = count >= 3072 ? 8 : count >= 2048 ? 4 : 1;
@@ -2470,6 +2470,7 @@ std::string autotune(int count, const sov_model* models, const sov_options* opt,
   const int sms = sm_count();
   for (size_t k = 0; k < B->buckets.size(); ++k) {
     auto& bk = B->buckets[k];
+    if (pinned_threads(bk->mmax)) continue;
     const int full = grid_for(bk->mmax, bk->threads, 1 << 30, 0) / sms;  // CTAs per SM that fit
     if (full < 2 || bk->count <= (full - 1) * sms) continue;             // nothing to trim
     const int old_g = bk->grid;
