@@ -73,7 +73,8 @@ enum {
 
 /* Normal-equation factorization (the reference's SOVEREIGN_IPM_NORMAL_EQUATIONS knob). */
 enum {
-  SOV_FACTOR_AUTO = 0,   /* banded when the bandwidth is small, else dense */
+  SOV_FACTOR_AUTO = 0,   /* banded when the bandwidth is small, else dense; sparse beyond the dense limit; a
+                            small LP as a batch of one (see sov_lp_solve) */
   SOV_FACTOR_DENSE = 1,  /* dense m x m Cholesky (dense-Schur) */
   SOV_FACTOR_BANDED = 2, /* banded LDL^T in the natural row order */
   SOV_FACTOR_XSPACE = 3, /* QP only: eliminate the slacks and factor Q + H + A'ZW^-1A over the structural
@@ -194,7 +195,13 @@ void sov_default_qp_options(sov_options* opt);
  * QP: qp_interior_point.cpp:155,195-197). */
 int sov_ipm_dims(const sov_model* model, int32_t qp, int32_t* n_ipm, int32_t* m_ipm);
 
-/* One LP through the GPU IPM. Synchronous; host pointers are borrowed for the call. */
+/* One LP through the GPU IPM. Synchronous; host pointers are borrowed for the call. A small LP in which no
+ * two rows share two columns (at most 128 IPM rows and 131072 entries, rows x entries at most 5 million: for
+ * instance transportation and assignment LPs) is solved as a batch of one, in one persistent launch and with the
+ * batched calls' process-lifetime buffers, streams and events; every other LP, and every LP for which
+ * diagnostics, an iterate on the way (ipm_iterate_at), mixed precision or a factorization is asked for, by the
+ * general engine, with buffers of the call's own. The two follow the same iteration with sums in another order, so
+ * asking for diagnostics can change an answer's last bits; each gives the same bits on every call. */
 int sov_lp_solve(const sov_model* model, const sov_options* opt, sov_result* result);
 
 /* One convex QP through the GPU IPM (QpInteriorPointSolver::solve, qp_interior_point.cpp:3123-3186).
@@ -211,7 +218,10 @@ int sov_qp_solve(const sov_model* model, const sov_options* opt, sov_result* res
  * of blocks opt_stride bytes apart, one per LP: per-LP tolerances, iteration limits, scaling and
  * warm starts (warm_x / warm_y / warm_s in the engine's standard form, taken under the same
  * safeguard as sov_lp_solve; diagnostics->warm_start_used reports it). LPs whose normal matrix
- * does not fit the batched kernel are solved one by one through sov_lp_solve. */
+ * does not fit the batched kernel are solved one by one by the general engine. The threads that work on an LP,
+ * and with them the order of its sums and an answer's last bits, follow from the number and sizes of the LPs in
+ * the call (or from sov_autotune); they do not follow from how a large call is cut into parts. An LP in which two
+ * rows share two columns can differ in the last bits between two calls. */
 int sov_lp_solve_batch(int32_t count, const sov_model* models, const sov_options* opt,
                        int32_t opt_stride, sov_result* results);
 
