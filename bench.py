@@ -231,8 +231,13 @@ def run_reference(args, rank: int, world: int):
         return
     from sovereign_b200 import problems as P
     import oracle
+    try:
+        threads = oracle.reference().ref_hardware_threads()
+    except OSError:
+        print(json.dumps(dict(impl="reference", unavailable="the reference library (oracle/_ref) is not built: its "
+                                                            "sources are not present")))
+        return
     models = P.transport_batch(COUNT, seed=2026)
-    threads = oracle.reference().ref_hardware_threads()
     # each step solves a bounded sample (about 4 s of CPU time) drawn round-robin from the batch
     probe = models[:threads]
     secs, *_ = oracle.solve_many_reference(probe, threads=threads)
